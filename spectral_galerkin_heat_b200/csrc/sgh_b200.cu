@@ -31,6 +31,7 @@
 #include "sgh_axis.cuh"
 #include "sgh_b200.h"
 #include "sgh_device.cuh"
+#include "sgh_fold.cuh"
 
 namespace {
 thread_local std::string g_last_error;
@@ -673,6 +674,135 @@ k_fs_commit_modes(const DevParams* __restrict__ P, double* a, const double* __re
   a[i] = a[i] * K[i] + kk * (Ct[z] * sigma[yx] + Cb[z] * beta[yx]);
 }
 
+// The face-space step without convection: volume pass -> face step in one
+// cluster (sgh_fold.cuh) -> volume pass.
+
+// Volume passes of the cluster form. Without COMMIT: the face sums of the
+// propagated modes aK = K a (Zt = sum Ct aK, Yt = sum aK KK Ct, per-block
+// partials of sum aK^2), for the first step of a launch; thread 0 also opens
+// the run. With COMMIT: a = K a + KK Ct sigma, and with SUMS the same face sums
+// of the new modes for the next step, so that the volume is read once per
+// step. A block takes 32 face columns and FV_Z z-planes at a time, FV_Z / 8 per
+// warp with all their loads in flight; warp 0 adds Zt plane by plane from
+// shared memory while the others load the next planes. Zt's order is that of
+// the batched volume pass, so that a plan and an FP64 batch slot stay equal bit
+// for bit; Yt and the norm (which only the convergence test reads) are added
+// warp by warp.
+constexpr int FV_COLS = 32, FV_Z = 64;
+template <bool COMMIT, bool SUMS>
+__global__ void __launch_bounds__(EW_THREADS)
+k_fs_volume(Ctrl* ctrl, sgh_laser laser, const sgh_laser* table, sgh_step_out* outs, int n_target, int nz, int S,
+            double* a, const double* __restrict__ K, const double* __restrict__ KK, const double* __restrict__ Ct,
+            const double* __restrict__ sigma, double* Zt, double* Yt, double* n1_parts) {
+  constexpr int NW = EW_THREADS / 32, U = FV_Z / NW;
+  __shared__ double sak[SUMS ? 2 : 1][SUMS ? FV_Z : 1][FV_COLS];
+  __shared__ double sh[2][NW][FV_COLS];
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  if (!COMMIT && blockIdx.x == 0 && threadIdx.x == 0) {
+    ctrl->laser = laser;
+    ctrl->table = table;
+    ctrl->out_table = outs;
+    ctrl->n_target = n_target;
+    ctrl->step = 0;
+  }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i = blockIdx.x * FV_COLS + lane;
+  const bool in = i < S;
+  double zt = 0.0, yt = 0.0, n1 = 0.0;
+  const double sg = COMMIT && in ? sigma[i] : 0.0;
+  for (int p0 = 0, buf = 0; p0 < nz; p0 += FV_Z, buf ^= 1) {
+    double av[U], kv[U], kk[U], ct[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int p = p0 + w + u * NW;
+      const bool ok = in && p < nz;
+      const size_t j = (size_t)(ok ? p : 0) * S + (in ? i : 0);
+      av[u] = ok ? a[j] : 0.0;
+      kv[u] = ok ? K[j] : 0.0;
+      kk[u] = ok ? KK[j] : 0.0;
+      ct[u] = p < nz ? Ct[p] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int p = p0 + w + u * NW;
+      double x = av[u];
+      if (COMMIT) {
+        x = __fma_rn(x, kv[u], __dmul_rn(kk[u], __dmul_rn(ct[u], sg)));
+        if (in && p < nz) a[(size_t)p * S + i] = x;
+      }
+      if (SUMS) {
+        const double ak = __dmul_rn(x, kv[u]);
+        sak[buf][w + u * NW][lane] = ak;
+        yt = fma(ak * kk[u], ct[u], yt);
+        n1 = fma(ak, ak, n1);
+      }
+    }
+    if (SUMS) {
+      __syncthreads();
+      if (w == 0)
+        for (int q = 0; q < FV_Z && p0 + q < nz; ++q) zt = fma(Ct[p0 + q], sak[buf][q][lane], zt);
+    }
+  }
+  if (!SUMS) return;
+  sh[0][w][lane] = yt;
+  sh[1][w][lane] = n1;
+  __syncthreads();
+  if (w == 0 && in) Zt[i] = zt;
+  if (w < 2) {
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < NW; ++q) s += sh[w][q][lane];
+    if (w == 1) {
+      s = fold::warp_sum(s);
+      if (lane == 0) n1_parts[blockIdx.x] = s;
+    } else if (in) {
+      Yt[i] = s;
+    }
+  }
+}
+
+// Step opening, Picard loop, surface commit and metrics of one instance in one
+// cluster (solvers/spectral.py:258-268, 273-306, 386-512, 536-542).
+__global__ void __launch_bounds__(fold::FACE_THREADS, 1)
+k_face_run(const DevParams* __restrict__ P, Ctrl* ctrl, fold::FaceShape f, fold::FaceJob<double> J,
+           cudaGraphConditionalHandle h_steps, int in_graph) {
+  extern __shared__ __align__(128) double fr_sh[];
+  __shared__ uint64_t bar[2];
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  const int step = ctrl->step;
+  const sgh_laser L = ctrl->table ? ctrl->table[step] : ctrl->laser;
+  const bool f32 = (L.flags & SGH_LASER_F32) != 0;
+  J.I0 = L.is_on ? P->absorptivity * L.power / (P->area_factor * (P->r_x * P->r_y)) : 0.0;
+  J.lx = L.x;
+  J.ly = L.y;
+  J.shift_x = laser_shift(L.vx, P->dt, P->dx, f32);
+  J.shift_y = laser_shift(L.vy, P->dt, P->dy, f32);
+  const bool ok = fold::face_operands(f, J, fr_sh, bar, umma::WAIT_LIMIT, false, &ctrl->umma_err);
+  const fold::FaceResult r = fold::face_step(f, J, fr_sh, !ok);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sgh_step_out o;
+    o.T_surface_max = r.tmax;
+    o.P_laser = r.qsum * P->dx * P->dy;
+    o.picard_rel_err = r.rel;
+    o.n_iter = r.iter;
+    o.converged = r.status == SGH_STEP_CONVERGED ? 1 : 0;
+    o.status = ctrl->umma_err ? SGH_STEP_TC_TIMEOUT : r.status;
+    o.flags = 0;
+    ctrl->laser = L;
+    ctrl->I0 = J.I0;
+    ctrl->shift_x = J.shift_x;
+    ctrl->shift_y = J.shift_y;
+    ctrl->iter = r.iter;
+    ctrl->stop = 1;
+    ctrl->status = r.status;
+    ctrl->rel_err = r.rel;
+    ctrl->out = o;
+    if (ctrl->out_table) ctrl->out_table[step] = o;
+    ctrl->step = step + 1;
+    if (in_graph) cudaGraphSetConditional(h_steps, step + 1 < ctrl->n_target ? 1u : 0u);
+  }
+}
+
 // Aligned sub-allocation of the caller's workspace.
 struct Layout {
   size_t off = 0;
@@ -703,6 +833,10 @@ struct sgh_plan {
   bool face_space = false;
   int nparts_fs = 0, nparts_n1 = 0;
   size_t o_fsF = 0, o_fsW = 0, o_sigma = 0, o_beta = 0, o_Ab = 0, o_pn1 = 0;
+  // cluster form of the face-space step (cluster = 0: not used): packed folded
+  // matrices (x forward, x inverse, y forward, y inverse) and volume partials
+  int cluster = 0;
+  size_t o_fold[4] = {0, 0, 0, 0}, o_pv = 0;
   // box mode: point-major x/y tables, z reconstruction (+ face row) and
   // projection matrices, window bases, pass scratch, source and history
   double box_z0 = 0.0;
@@ -1002,6 +1136,44 @@ void enqueue_picard_face_space(sgh_plan* p, cudaStream_t s, cudaGraphConditional
   ++g_launches;
 }
 
+fold::FaceJob<double> face_job(sgh_plan* p) {
+  const DevParams& h = p->hp;
+  fold::FaceJob<double> J = {};
+  J.cell_integrated = h.cell_integrated;
+  J.dx = h.dx; J.dy = h.dy; J.r_x = h.r_x; J.r_y = h.r_y; J.order = h.order;
+  J.T_liquidus = h.T_liquidus; J.T_boil = h.T_boil; J.evap_f1 = h.evap_f1; J.evap_f2 = h.evap_f2;
+  J.dct_scale = h.dct_scale; J.recon_scale = h.recon_scale; J.omega = h.omega; J.tol = h.tol;
+  J.n_elements = h.n_elements;
+  J.max_iter = h.max_iter;
+  J.pxf = p->d(p->o_fold[0]); J.pxi = p->d(p->o_fold[1]);
+  J.pyf = p->d(p->o_fold[2]); J.pyi = p->d(p->o_fold[3]);
+  J.Zt = p->d(p->o_fsF); J.Yt = p->d(p->o_fsF) + 2 * (size_t)h.S;
+  J.Wtt = p->d(p->o_fsW); J.Qtt = p->d(p->o_fsW) + 3 * (size_t)h.S;
+  J.part_n1 = p->d(p->o_pv);
+  J.n_n1 = cdiv(h.S, FV_COLS);
+  J.qlas = p->d(p->o_qlas); J.qev = p->d(p->o_qevold); J.sigma = p->d(p->o_sigma); J.Tsurf = p->d(p->o_Tsurf);
+  J.hist = p->d(p->o_hist);
+  J.hist_cap = p->hist_cap;
+  return J;
+}
+
+// Volume pass of the cluster form (see k_fs_volume).
+template <bool COMMIT, bool SUMS>
+void enqueue_fs_volume(sgh_plan* p, cudaStream_t s, const sgh_laser& laser, const sgh_laser* table,
+                       sgh_step_out* outs, int n) {
+  const DevParams& h = p->hp;
+  launch_pdl(k_fs_volume<COMMIT, SUMS>, dim3(cdiv(h.S, FV_COLS)), EW_THREADS, 0, s, p->ctrl(), laser, table, outs, n,
+             h.nz, h.S, p->d(p->o_a), p->d(p->o_K), p->d(p->o_KK), p->d(p->o_ct), p->d(p->o_sigma), p->d(p->o_fsF),
+             p->d(p->o_fsF) + 2 * (size_t)h.S, p->d(p->o_pv));
+  ++g_launches;
+}
+void enqueue_face_run(sgh_plan* p, cudaStream_t s, cudaGraphConditionalHandle h_steps, int in_graph) {
+  const fold::FaceShape f = fold::face_shape<double>(p->hp.nx, p->hp.ny, p->cluster);
+  SGH_CK_VOID(fold::launch_cluster(k_face_run, f.n, f.n, fold::threads_for(f), f.bytes, true, s, p->P(), p->ctrl(), f, face_job(p), h_steps,
+                                   in_graph));
+  ++g_launches;
+}
+
 // BF16 pair plane of one matrix of a mixed plan.
 void build_plane(sgh_plan* p, const sgh_plan::PlaneSpec& q, cudaStream_t s) {
   const long n = (long)cdiv(q.rows, AXU_M) * AXU_M * (long)cdiv(q.k, AXU_KC) * AXU_KC;
@@ -1225,6 +1397,15 @@ void enqueue_post(sgh_plan* p, cudaStream_t s, cudaGraphConditionalHandle h_step
   ++g_launches;
 }
 
+// Cluster size of the face-space step, or 0 for the multi-kernel form
+// (convection, reduced precision, faces too large for a cluster).
+int face_cluster(const sgh_plan* p) {
+  const DevParams& h = p->hp;
+  if (!p->face_space || h.has_top_conv || h.has_bottom_conv) return 0;
+  if (p->cfg.precision != SGH_PRECISION_FP64) return 0;
+  return fold::cluster_size<double>(h.nx, h.ny);
+}
+
 // Adds a conditional node of the given type to the graph being captured on
 // cs (after the captured work so far) and returns its body graph.
 int add_conditional(cudaStream_t cs, cudaGraphConditionalHandle h, cudaGraphConditionalNodeType type,
@@ -1262,6 +1443,19 @@ int capture(sgh_plan* p) {
   cudaGraph_t body = outer.conditional.phGraph_out[0];
 
   SGH_CK(cudaStreamBeginCaptureToGraph(p->cs1, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+  if (p->cluster) {  // the first step's face sums are launched ahead of the graph (begin_run)
+    g_launches = 0;
+    enqueue_face_run(p, p->cs1, h_steps, 1);
+    p->n_pre = g_launches;
+    p->n_iter = 0;
+    g_launches = 0;
+    enqueue_fs_volume<true, true>(p, p->cs1, sgh_laser{}, nullptr, nullptr, 0);
+    p->n_post = g_launches;
+    SGH_CK(cudaStreamEndCapture(p->cs1, &body));
+    SGH_CK(cudaGetLastError());
+    SGH_CK(cudaGraphInstantiate(&p->exec, G, 0));
+    return SGH_OK;
+  }
   cudaGraphConditionalHandle h_picard, h_seed = 0;
   SGH_CK(cudaGraphConditionalHandleCreate(&h_picard, body, 0, 0));
   if (p->hp.box) SGH_CK(cudaGraphConditionalHandleCreate(&h_seed, body, 0, 0));
@@ -1508,6 +1702,11 @@ int sgh_plan_create(const sgh_config* cfg, sgh_plan** out) {
   p->o_beta = L.take(S8);
   p->o_Ab = L.take(S8);
   p->o_pn1 = L.take(sizeof(double) * p->nparts_n1);
+  p->cluster = face_cluster(p);
+  if (p->cluster) {
+    for (int q = 0; q < 4; ++q) p->o_fold[q] = L.take(sizeof(double) * fold::pack_doubles(q < 2 ? h.nx : h.ny));
+    p->o_pv = L.take(sizeof(double) * cdiv(h.S, FV_COLS));
+  }
   if (c.precision == SGH_PRECISION_MIXED) {
     // each matrix with the largest (rows, contraction length) its passes use
     auto plane = [&](size_t mat, int rows, int k, bool per_step = false) {
@@ -1587,6 +1786,12 @@ int sgh_plan_bind(sgh_plan* p, void* workspace, uint64_t bytes, void* stream) {
     SGH_CK(cudaMemcpyAsync(p->d(p->o_bzi) + (size_t)h.zb * h.nz, p->d(p->o_ct), sizeof(double) * h.nz,
                            cudaMemcpyDeviceToDevice, s));
   }
+  if (p->cluster)
+    for (int q = 0; q < 2; ++q) {
+      const int N = q ? h.ny : h.nx;
+      fold::k_fold_pack<<<std::min(cdiv((long)fold::pack_doubles(N), EW_THREADS), 1184), EW_THREADS, 0, s>>>(
+          N, p->d(q ? p->o_my : p->o_mx), p->d(p->o_fold[2 * q]), p->d(p->o_fold[2 * q + 1]));
+    }
   if (p->face_space)
     k_fs_weights<<<cdiv(h.S, EW_THREADS), EW_THREADS, 0, s>>>(p->P(), p->d(p->o_KK), p->d(p->o_ct),
                                                               p->d(p->o_cb), p->d(p->o_fsW));
@@ -1684,6 +1889,15 @@ int sgh_step(sgh_plan* p, const sgh_laser* laser, sgh_step_out* out, void* strea
   if (!p || !laser) return fail(SGH_ERR_INVALID, "null argument");
   if (!p->bound) return fail(SGH_ERR_STATE, "plan is not bound");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (p->cluster) {  // three launches: cheaper than a graph with a conditional node
+    enqueue_fs_volume<false, true>(p, s, *laser, nullptr, nullptr, 1);
+    enqueue_face_run(p, s, 0, 0);
+    enqueue_fs_volume<true, false>(p, s, sgh_laser{}, nullptr, nullptr, 0);
+    SGH_CK(cudaGetLastError());
+    if (out) SGH_CK(cudaMemcpyAsync(out, &p->ctrl()->out, sizeof(sgh_step_out), cudaMemcpyDeviceToHost, s));
+    SGH_CK(cudaStreamSynchronize(s));
+    return SGH_OK;
+  }
   k_run_setup<<<1, 1, 0, s>>>(p->ctrl(), *laser, nullptr, nullptr, 1);
   SGH_CK(cudaGetLastError());
   SGH_CK(cudaGraphLaunch(p->exec, s));
@@ -1697,6 +1911,7 @@ int sgh_step_eager(sgh_plan* p, const sgh_laser* laser, sgh_step_out* out, void*
                     plan_fp32(p), planes_of(p), nplanes_of(p));
   if (!p || !laser) return fail(SGH_ERR_INVALID, "null argument");
   if (!p->bound) return fail(SGH_ERR_STATE, "plan is not bound");
+  if (p->cluster) return sgh_step(p, laser, out, stream);  // its kernels are launched one by one already
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   k_run_setup<<<1, 1, 0, s>>>(p->ctrl(), *laser, nullptr, nullptr, 1);
   enqueue_pre(p, s);
@@ -1721,7 +1936,10 @@ int sgh_run(sgh_plan* p, const sgh_laser* lasers_dev, int32_t n_steps, sgh_step_
   if (n_steps == 0) return SGH_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   sgh_laser dummy = {};
-  k_run_setup<<<1, 1, 0, s>>>(p->ctrl(), dummy, lasers_dev, outs_dev, n_steps);
+  if (p->cluster)
+    enqueue_fs_volume<false, true>(p, s, dummy, lasers_dev, outs_dev, n_steps);
+  else
+    k_run_setup<<<1, 1, 0, s>>>(p->ctrl(), dummy, lasers_dev, outs_dev, n_steps);
   SGH_CK(cudaGetLastError());
   SGH_CK(cudaGraphLaunch(p->exec, s));
   return SGH_OK;

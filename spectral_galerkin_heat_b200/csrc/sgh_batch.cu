@@ -34,6 +34,7 @@
 #include "sgh_b200.h"
 #include "sgh_axis.cuh"
 #include "sgh_device.cuh"
+#include "sgh_fold.cuh"
 #include "sgh_umma.cuh"
 
 namespace sgh {
@@ -65,6 +66,8 @@ struct BSlot {
   long long mpx, mpy;  // byte offsets of the forward x / y matrix planes (inverse at + mp_inv)
   long long mpx_inv, mpy_inv;
   long long x1;        // byte offset of the slot's x1 plane (x-pass result, y-pass B operand)
+  int cl, pad_cl;      // CTAs of the slot's cluster (kb_face_cluster); 0: the multi-kernel face path
+  long long fold[4];   // element offsets of the packed matrices: x forward, x inverse, y forward, y inverse
   double dx, dy, dt, Lx, Ly, Lz;
   double dct_scale, recon_scale, n_elements;
   double T0, evap_f1, evap_f2, T_boil, T_liquidus;
@@ -83,6 +86,7 @@ struct BState {
   int pass1_ready;   // the commit already formed the next step's face sums
   int pad2;
   double I0, shift_x, shift_y, rel_err;
+  double qsum, tmax;  // sum of q_las and surface maximum of the step (cluster slots)
   sgh_step_out last;
 };
 
@@ -347,7 +351,7 @@ __global__ void __launch_bounds__(CT) kb_begin(BView v, cudaGraphConditionalHand
     st.iter = 0;
     st.status = SGH_STEP_CAPPED;
     st.rel_err = nan("");
-    st.done = sl.max_iter > 0 ? 0 : 1;
+    st.done = sl.max_iter > 0 && !sl.cl ? 0 : 1;  // cluster slots run their Picard loop in one kernel
     st.tickets = 0u;
     if (!st.done) atomicAdd(&any, 1);
   }
@@ -1161,6 +1165,55 @@ kb_relax(BView v, const double* Zt, const double* Yt, const double* Wtt, const d
   relax_finish<BT>(v, s, b, sl.rblk0, sl.nrblk, r2, o2, part, part_n1, h_picard, in_graph, sh);
 }
 
+// Face step of the slots whose face runs in one cluster (sgh_fold.cuh): laser
+// flux and warm start, the Picard loop with its convergence test, the surface
+// commit. The slots of `list` take cl CTAs each, shape[s] giving the division
+// of slot s. FP64 contractions in either precision.
+struct FaceArrays {
+  const void *Zt, *Yt, *Wtt, *Qtt;
+  const double* part_n1;
+  double *qlas, *qev, *sigma, *Tsurf;
+  const double* fold;
+};
+template <class W>
+__global__ void __launch_bounds__(fold::FACE_THREADS, 1)
+kb_face_cluster(BView v, const int* list, const fold::FaceShape* shape, int cl, FaceArrays q) {
+  extern __shared__ __align__(128) double fc_sh[];
+  __shared__ uint64_t bar[2];
+  const int s = list[blockIdx.x / cl];
+  const BSlot& sl = v.slot[s];
+  BState& st = v.st[s];
+  if (!st.active) return;
+  const fold::FaceShape f = shape[s];
+  fold::FaceJob<W> J;
+  J.cell_integrated = sl.cell_integrated;
+  J.dx = sl.dx; J.dy = sl.dy; J.r_x = sl.r_x; J.r_y = sl.r_y; J.order = sl.order;
+  J.T_liquidus = sl.T_liquidus; J.T_boil = sl.T_boil; J.evap_f1 = sl.evap_f1; J.evap_f2 = sl.evap_f2;
+  J.dct_scale = sl.dct_scale; J.recon_scale = sl.recon_scale; J.omega = sl.omega; J.tol = sl.tol;
+  J.n_elements = sl.n_elements;
+  J.max_iter = sl.max_iter;
+  J.I0 = st.I0; J.lx = st.laser.x; J.ly = st.laser.y; J.shift_x = st.shift_x; J.shift_y = st.shift_y;
+  J.pxf = q.fold + sl.fold[0]; J.pxi = q.fold + sl.fold[1];
+  J.pyf = q.fold + sl.fold[2]; J.pyi = q.fold + sl.fold[3];
+  J.Zt = static_cast<const W*>(q.Zt) + sl.face; J.Yt = static_cast<const W*>(q.Yt) + sl.face;
+  J.Wtt = static_cast<const W*>(q.Wtt) + sl.face; J.Qtt = static_cast<const W*>(q.Qtt) + sl.face;
+  J.part_n1 = q.part_n1 + sl.blk0;
+  J.n_n1 = sl.nblk;
+  J.qlas = q.qlas + sl.face; J.qev = q.qev + sl.face; J.sigma = q.sigma + sl.face; J.Tsurf = q.Tsurf + sl.face;
+  J.hist = nullptr;
+  J.hist_cap = 0;
+  const unsigned lim = v.g->wait_limit ? v.g->wait_limit : umma::WAIT_LIMIT;
+  const bool ok = fold::face_operands(f, J, fc_sh, bar, lim, v.g->stall_test != 0, &v.g->umma_err);
+  const fold::FaceResult r = fold::face_step(f, J, fc_sh, !ok);
+  if (blockIdx.x % cl == 0 && threadIdx.x == 0) {
+    st.iter = r.iter;
+    st.status = r.status;
+    st.rel_err = r.rel;
+    st.qsum = r.qsum;
+    st.tmax = r.tmax;
+  }
+}
+
 // ---- volume passes ----------------------------------------------------------
 // One thread per VEC consecutive (y, x) columns of a slot, looping over z;
 // a, K and KK move as VEC-wide vectors (the slot's volume offset and face
@@ -1302,8 +1355,9 @@ kb_volume(BView v, R* a, const R* K, const R* KK, const double* sigma, R* Zt, R*
             for (int c = 0; c < VEC; ++c) {
               const double kv = (double)kvv[u][c];
               const double kk = (double)kkv[u][c];
-              if (COMMIT) av[u][c] = (R)((double)av[u][c] * kv + kk * (cp * sg[c]));
-              const double ak = (double)av[u][c] * kv;
+              // rounded as k_fs_volume (sgh_b200.cu) rounds it, so that a slot equals a plan
+              if (COMMIT) av[u][c] = (R)__fma_rn((double)av[u][c], kv, __dmul_rn(kk, __dmul_rn(cp, sg[c])));
+              const double ak = __dmul_rn((double)av[u][c], kv);
               zt[c] = fma(cp, ak, zt[c]);
               yt[c] = fma(ak * kk, cp, yt[c]);
               n1 = fma(ak, ak, n1);
@@ -1494,6 +1548,10 @@ kb_commit(BView v, const double* part_las, const double* part_tile, int umma_til
     if (!st.active) continue;
     const BSlot& sl = v.slot[s];
     double p = 0.0, m = -INFINITY;
+    if (sl.cl) {
+      p = lane == 0 ? st.qsum : 0.0;
+      m = st.tmax;
+    }
     for (int b = sl.rblk0 + lane; b < sl.rblk0 + sl.nrblk; b += 32) p += part_las[b];
     const int t0 = umma_tiles ? sl.utile0 : sl.tile0, nt = umma_tiles ? sl.nutile : sl.ntile;
     for (int b = t0 + lane; b < t0 + nt; b += 32) m = fmax(m, part_tile[b]);
@@ -1549,6 +1607,19 @@ struct sgh_batch {
   size_t o_qlas, o_qnet, o_qevold, o_Stop, o_f1, o_sigma, o_A, o_Tsurf, o_Zt, o_Yt, o_Wtt, o_Qtt;
   size_t o_plas, o_pn1, o_prelax, o_ptile;
   size_t o_xa = 0, o_xq = 0, o_mp = 0, o_x1 = 0;  // operand pair planes (mixed)
+  // slots whose face runs in one cluster, by cluster size (largest first):
+  // launch groups over clist, per-slot shapes, packed folded matrices
+  struct ClusterGroup {
+    int n, first, count, threads, bytes;
+  };
+  std::vector<ClusterGroup> cgroups;
+  cudaStream_t gs[5] = {};  // streams and events of the groups beyond the first
+  cudaEvent_t ge[5] = {};
+  std::vector<int> clist;
+  std::vector<fold::FaceShape> cshape;
+  std::vector<std::pair<int, long long>> fold_list;  // (N, element offset: forward, inverse)
+  long long fold_elems = 0;
+  size_t o_clist = 0, o_cshape = 0, o_fold = 0;
   size_t xa_bytes = 0, mp_bytes = 0, x1_bytes = 0;
   int vec = 1;  // columns per thread of the volume passes
   int vol_unroll = 4;  // z-planes per load round of the volume passes (2, 4 or 8)
@@ -1655,19 +1726,50 @@ void launch_volume(sgh_batch* B, cudaStream_t s, R* a, const R* K, const R* KK) 
   else with_u(std::integral_constant<int, 1>{});
 }
 
+// Whether some slot takes the multi-kernel face path.
+bool has_wide(const sgh_batch* B) { return B->tot_rblk > 0; }
+
+// The face steps of the cluster slots, one launch per cluster size.
+template <class R>
+void enqueue_clusters(sgh_batch* B, cudaStream_t s) {
+  FaceArrays q;
+  q.Zt = B->ws + B->o_Zt; q.Yt = B->ws + B->o_Yt; q.Wtt = B->ws + B->o_Wtt; q.Qtt = B->ws + B->o_Qtt;
+  q.part_n1 = B->d(B->o_pn1);
+  q.qlas = B->d(B->o_qlas); q.qev = B->d(B->o_qevold); q.sigma = B->d(B->o_sigma); q.Tsurf = B->d(B->o_Tsurf);
+  q.fold = B->d(B->o_fold);
+  // the groups run side by side: the first on s, the others on streams forked
+  // from it and joined again
+  const int ng = (int)B->cgroups.size();
+  for (int k = 0; k < ng; ++k) {
+    const auto& g = B->cgroups[k];
+    cudaStream_t t = k ? B->gs[k] : s;
+    if (k == 0 && ng > 1) (void)cudaEventRecord(B->ge[0], s);
+    if (k) (void)cudaStreamWaitEvent(t, B->ge[0], 0);
+    (void)fold::launch_cluster(kb_face_cluster<R>, g.n * g.count, g.n, g.threads, g.bytes, false, t, B->view(),
+                               reinterpret_cast<const int*>(B->ws + B->o_clist) + g.first,
+                               reinterpret_cast<const fold::FaceShape*>(B->ws + B->o_cshape), g.n, q);
+    g_blaunch += 1;
+    if (k) (void)cudaEventRecord(B->ge[k], t);
+  }
+  for (int k = 1; k < ng; ++k) (void)cudaStreamWaitEvent(s, B->ge[k], 0);
+}
+
 template <class R>
 void enqueue_pre(sgh_batch* B, cudaStream_t s, cudaGraphConditionalHandle h, int in_graph) {
   const BView v = B->view();
   R* a = reinterpret_cast<R*>(B->ws + B->o_a);
   R* K = B->precision == SGH_PRECISION_MIXED ? nullptr : reinterpret_cast<R*>(B->ws + B->o_K);
   R* KK = B->precision == SGH_PRECISION_MIXED ? nullptr : reinterpret_cast<R*>(B->ws + B->o_KK);
-  kb_begin<<<1, CT, 0, s>>>(v, h, in_graph);
+  const bool wide = has_wide(B);
+  kb_begin<<<1, CT, 0, s>>>(v, h, in_graph && wide);
   // mixed precision: q_net goes only into the operand plane of the transform
-  kb_face_begin<<<B->tot_rblk, BT, 0, s>>>(v, B->d(B->o_qlas),
+  if (wide) kb_face_begin<<<B->tot_rblk, BT, 0, s>>>(v, B->d(B->o_qlas),
                                            B->precision == SGH_PRECISION_MIXED ? nullptr : B->d(B->o_qnet),
                                            B->d(B->o_qevold), B->d(B->o_plas));
   launch_volume<R, false>(B, s, a, K, KK);
-  g_blaunch += 3;
+  g_blaunch += wide ? 3 : 2;
+  enqueue_clusters<R>(B, s);
+  if (!wide) return;
   // initial guess: sigma = dct_scale * DCT2(q_las - shift(q_evap_old)), then A = Zt + W_tt sigma
   if (B->precision == SGH_PRECISION_MIXED) {
     face2d<false, false, F2_SIGMA>(B, s, B->d(B->o_qnet), EB_Store{B->d(B->o_sigma), 1},
@@ -1707,7 +1809,8 @@ void enqueue_post(sgh_batch* B, cudaStream_t s, cudaGraphConditionalHandle h, in
   R* a = reinterpret_cast<R*>(B->ws + B->o_a);
   R* K = B->precision == SGH_PRECISION_MIXED ? nullptr : reinterpret_cast<R*>(B->ws + B->o_K);
   R* KK = B->precision == SGH_PRECISION_MIXED ? nullptr : reinterpret_cast<R*>(B->ws + B->o_KK);
-  face2d<true, false, F2_COMMIT>(B, s, B->d(B->o_A),
+  if (has_wide(B))
+    face2d<true, false, F2_COMMIT>(B, s, B->d(B->o_A),
                                  EB_CommitSurface{B->d(B->o_Tsurf)},
                                  F2Args{B->d(B->o_Tsurf), nullptr, nullptr, 0}, B->d(B->o_ptile));
   launch_volume<R, true>(B, s, a, K, KK);
@@ -1732,30 +1835,33 @@ int capture(sgh_batch* B) {
   SGB_CK(cudaGraphAddNode(&outer_node, G, nullptr, 0, &outer));
   cudaGraph_t body = outer.conditional.phGraph_out[0];
   SGB_CK(cudaStreamBeginCaptureToGraph(B->cs1, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-  cudaGraphConditionalHandle h_picard;
-  SGB_CK(cudaGraphConditionalHandleCreate(&h_picard, body, 0, 0));
+  cudaGraphConditionalHandle h_picard = 0;
+  if (has_wide(B)) SGB_CK(cudaGraphConditionalHandleCreate(&h_picard, body, 0, 0));
   g_blaunch = 0;
   enqueue_pre<R>(B, B->cs1, h_picard, 1);
   B->n_pre = g_blaunch;
-  cudaStreamCaptureStatus status;
-  cudaGraph_t cur;
-  const cudaGraphNode_t* deps = nullptr;
-  size_t ndeps = 0;
-  SGB_CK(cudaStreamGetCaptureInfo(B->cs1, &status, nullptr, &cur, &deps, &ndeps));
-  cudaGraphNodeParams inner = {};
-  inner.type = cudaGraphNodeTypeConditional;
-  inner.conditional.handle = h_picard;
-  inner.conditional.type = cudaGraphCondTypeWhile;
-  inner.conditional.size = 1;
-  cudaGraphNode_t inner_node;
-  SGB_CK(cudaGraphAddNode(&inner_node, cur, deps, ndeps, &inner));
-  SGB_CK(cudaStreamUpdateCaptureDependencies(B->cs1, &inner_node, 1, cudaStreamSetCaptureDependencies));
-  cudaGraph_t ibody = inner.conditional.phGraph_out[0];
-  SGB_CK(cudaStreamBeginCaptureToGraph(B->cs2, ibody, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-  g_blaunch = 0;
-  enqueue_picard(B, B->cs2, h_picard, 1);
-  B->n_iter = g_blaunch;
-  SGB_CK(cudaStreamEndCapture(B->cs2, &ibody));
+  B->n_iter = 0;
+  if (has_wide(B)) {  // cluster slots iterate inside their kernel
+    cudaStreamCaptureStatus status;
+    cudaGraph_t cur;
+    const cudaGraphNode_t* deps = nullptr;
+    size_t ndeps = 0;
+    SGB_CK(cudaStreamGetCaptureInfo(B->cs1, &status, nullptr, &cur, &deps, &ndeps));
+    cudaGraphNodeParams inner = {};
+    inner.type = cudaGraphNodeTypeConditional;
+    inner.conditional.handle = h_picard;
+    inner.conditional.type = cudaGraphCondTypeWhile;
+    inner.conditional.size = 1;
+    cudaGraphNode_t inner_node;
+    SGB_CK(cudaGraphAddNode(&inner_node, cur, deps, ndeps, &inner));
+    SGB_CK(cudaStreamUpdateCaptureDependencies(B->cs1, &inner_node, 1, cudaStreamSetCaptureDependencies));
+    cudaGraph_t ibody = inner.conditional.phGraph_out[0];
+    SGB_CK(cudaStreamBeginCaptureToGraph(B->cs2, ibody, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    g_blaunch = 0;
+    enqueue_picard(B, B->cs2, h_picard, 1);
+    B->n_iter = g_blaunch;
+    SGB_CK(cudaStreamEndCapture(B->cs2, &ibody));
+  }
   g_blaunch = 0;
   enqueue_post<R>(B, B->cs1, h_steps, 1);
   B->n_post = g_blaunch;
@@ -1763,6 +1869,22 @@ int capture(sgh_batch* B) {
   SGB_CK(cudaGetLastError());
   SGB_CK(cudaGraphInstantiate(&B->exec, G, 0));
   return SGH_OK;
+}
+
+// CTAs of the cluster that runs a slot's face step, 0 for the multi-kernel path.
+// A rule on the slot's own shape and Picard cap, so that its results do not
+// depend on the rest of the batch. FP64: wherever the face fits (18 serving
+// slots up to 256 x 128: 1.71 -> 0.86 ms for 6 steps). Mixed: Picard loops up to
+// 32768 elements, where the launches and epilogue latencies of the tensor-core
+// kernels dominate (32 uneven slots, 3 steps of 30 iterations: 7.6 -> 2.4 ms; 4
+// small ragged slots: 10.3 -> 1.9 ms); with one forcing pass per step the
+// tensor-core kernels take all slots of a batch at once and are faster (48
+// serving slots: 1.45 ms against 1.50 with the 64 x 32 faces on clusters, 1.85
+// with every face up to 256 x 128).
+int slot_cluster(const sgh_config& c, int precision) {
+  if (precision != SGH_PRECISION_MIXED) return fold::cluster_size<double>(c.nx, c.ny);
+  if (c.max_iter <= 1 || (long)c.nx * c.ny > 32768) return 0;
+  return fold::cluster_size<float>(c.nx, c.ny);
 }
 
 struct LayoutB {
@@ -1827,7 +1949,10 @@ int sgh_batch_create(const sgh_config* cfgs, int32_t n, int32_t precision, sgh_b
   std::map<int, long long> mplane;
   if (precision == SGH_PRECISION_MIXED) {
     long long po = 0;
-    for (auto& kv : mats) {
+    std::map<int, int> wide;  // lengths of the slots on the tensor-core path
+    for (int i = 0; i < n; ++i)
+      if (!slot_cluster(cfgs[i], precision)) wide[cfgs[i].nx] = wide[cfgs[i].ny] = 1;
+    for (auto& kv : wide) {
       // per N: forward, inverse in 128-row chunks (the A operand of the
       // y-pass and the B operand of the x-pass alike)
       mplane[kv.first] = po;
@@ -1836,6 +1961,14 @@ int sgh_batch_create(const sgh_config* cfgs, int32_t n, int32_t precision, sgh_b
     }
     B->mp_bytes = (size_t)po;
   }
+  auto fold_at = [&](int N) {  // offset of the packed matrices of length N
+    for (const auto& q : B->fold_list)
+      if (q.first == N) return q.second;
+    const long long o = B->fold_elems;
+    B->fold_list.push_back({N, o});
+    B->fold_elems += 2 * (long long)fold::pack_doubles(N);
+    return o;
+  };
   for (int i = 0; i < n; ++i) {
     const sgh_config& c = cfgs[i];
     BSlot sl;
@@ -1852,13 +1985,16 @@ int sgh_batch_create(const sgh_config* cfgs, int32_t n, int32_t precision, sgh_b
     sl.mx = (int)mats[c.nx];
     sl.my = (int)mats[c.ny];
     sl.nblk = cdivl(sl.S, BT);
+    sl.cl = slot_cluster(c, precision);
+    if (sl.cl)
+      for (int q = 0; q < 4; ++q) sl.fold[q] = fold_at(q < 2 ? c.nx : c.ny) + (q & 1) * (long long)fold::pack_doubles(q < 2 ? c.nx : c.ny);
     sl.rblk0 = B->tot_rblk;
-    sl.nrblk = cdivl(sl.S, RB);
-    sl.ntile = face_tiles(c.nx, c.ny);
+    sl.nrblk = sl.cl ? 0 : cdivl(sl.S, RB);
+    sl.ntile = sl.cl ? 0 : face_tiles(c.nx, c.ny);
     sl.vblk0 = B->tot_vblk;
     sl.nvblk = cdivl(sl.V, BT);
-    sl.nutile = face_utiles(c.nx, c.ny);
-    if (precision == SGH_PRECISION_MIXED) {
+    sl.nutile = sl.cl ? 0 : face_utiles(c.nx, c.ny);
+    if (precision == SGH_PRECISION_MIXED && !sl.cl) {
       sl.xa = (long long)B->xa_bytes;
       B->xa_bytes += umma::pair_bytes<128>(c.ny, c.nx);
       sl.x1 = (long long)B->x1_bytes;
@@ -1928,6 +2064,24 @@ int sgh_batch_create(const sgh_config* cfgs, int32_t n, int32_t precision, sgh_b
       B->utile_slot.insert(B->utile_slot.end(), sl.nutile, i);
     }
   }
+  B->cshape.resize(n);
+  for (int cl = fold::FACE_MAX_CLUSTER; cl >= 1; cl /= 2) {
+    sgh_batch::ClusterGroup g = {cl, (int)B->clist.size(), 0, 0, 0};
+    std::vector<int> m;
+    for (int i = 0; i < n; ++i)
+      if (B->slots[i].cl == cl) m.push_back(i);
+    std::stable_sort(m.begin(), m.end(), [&](int a, int b) { return B->slots[a].S > B->slots[b].S; });
+    for (int i : m) {
+      const BSlot& sl = B->slots[i];
+      B->cshape[i] = precision == SGH_PRECISION_MIXED ? fold::face_shape<float>(sl.nx, sl.ny, cl)
+                                                      : fold::face_shape<double>(sl.nx, sl.ny, cl);
+      g.threads = std::max(g.threads, fold::threads_for(B->cshape[i]));
+      g.bytes = std::max(g.bytes, B->cshape[i].bytes);
+    }
+    g.count = (int)m.size();
+    B->clist.insert(B->clist.end(), m.begin(), m.end());
+    if (g.count) B->cgroups.push_back(g);
+  }
   {
     const int vw = precision == SGH_PRECISION_MIXED ? 4 : 2;
     bool ok = true;
@@ -1977,6 +2131,11 @@ int sgh_batch_create(const sgh_config* cfgs, int32_t n, int32_t precision, sgh_b
     B->o_mp = L.take(B->mp_bytes);
     B->o_x1 = L.take(B->x1_bytes);
   }
+  if (!B->clist.empty()) {
+    B->o_clist = L.take(sizeof(int) * B->clist.size());
+    B->o_cshape = L.take(sizeof(fold::FaceShape) * (size_t)n);
+    B->o_fold = L.take(sizeof(double) * (size_t)B->fold_elems);
+  }
   B->ws_need = L.off;
   *out = B;
   return SGH_OK;
@@ -1988,6 +2147,10 @@ int sgh_batch_destroy(sgh_batch* B) {
   if (B->graph) cudaGraphDestroy(B->graph);
   if (B->cs1) cudaStreamDestroy(B->cs1);
   if (B->cs2) cudaStreamDestroy(B->cs2);
+  for (int k = 0; k < 5; ++k) {
+    if (B->gs[k]) cudaStreamDestroy(B->gs[k]);
+    if (B->ge[k]) cudaEventDestroy(B->ge[k]);
+  }
   delete B;
   return SGH_OK;
 }
@@ -2029,6 +2192,7 @@ int sgh_batch_bind(sgh_batch* B, void* workspace, uint64_t bytes, void* stream) 
   SGB_CK(cudaMemsetAsync(B->ws + B->o_state, 0, sizeof(BState) * n, s));
   SGB_CK(cudaMemsetAsync(B->ws + B->o_g, 0, sizeof(BGlobal), s));
   const auto put = [&](size_t off, const std::vector<int>& m) {
+    if (m.empty()) return cudaSuccess;
     return cudaMemcpyAsync(B->ws + off, m.data(), sizeof(int) * m.size(), cudaMemcpyHostToDevice, s);
   };
   SGB_CK(put(B->o_blk, B->blk_slot));
@@ -2039,6 +2203,18 @@ int sgh_batch_bind(sgh_batch* B, void* workspace, uint64_t bytes, void* stream) 
   SGB_CK(cudaMemsetAsync(B->ws + B->o_qevold, 0, sizeof(double) * B->tot_face, s));
   for (auto& m : B->mat_list)
     kb_dct_matrix<<<cdivl((long long)m.first * m.first, BT), BT, 0, s>>>(m.first, B->d(B->o_mats) + m.second);
+  if (!B->clist.empty()) {
+    SGB_CK(put(B->o_clist, B->clist));
+    SGB_CK(cudaMemcpyAsync(B->ws + B->o_cshape, B->cshape.data(), sizeof(fold::FaceShape) * n,
+                           cudaMemcpyHostToDevice, s));
+    for (const auto& q : B->fold_list) {
+      const long m = (long)fold::pack_doubles(q.first);
+      double* o = B->d(B->o_fold) + q.second;
+      for (const auto& mt : B->mat_list)
+        if (mt.first == q.first)
+          fold::k_fold_pack<<<std::min(cdivl(m, BT), 1184), BT, 0, s>>>(q.first, B->d(B->o_mats) + mt.second, o, o + m);
+    }
+  }
   const BView v = B->view();
   if (B->precision == SGH_PRECISION_MIXED) {
     SGB_CK(cudaMemsetAsync(B->ws + B->o_xa, 0, B->xa_bytes, s));
@@ -2069,6 +2245,10 @@ int sgh_batch_bind(sgh_batch* B, void* workspace, uint64_t bytes, void* stream) 
   SGB_CK(cudaStreamSynchronize(s));
   SGB_CK(cudaStreamCreateWithFlags(&B->cs1, cudaStreamNonBlocking));
   SGB_CK(cudaStreamCreateWithFlags(&B->cs2, cudaStreamNonBlocking));
+  for (size_t k = 0; k < B->cgroups.size() && B->cgroups.size() > 1; ++k) {
+    if (k) SGB_CK(cudaStreamCreateWithFlags(&B->gs[k], cudaStreamNonBlocking));
+    SGB_CK(cudaEventCreateWithFlags(&B->ge[k], cudaEventDisableTiming));
+  }
   const int rc = B->precision == SGH_PRECISION_MIXED ? capture<float>(B) : capture<double>(B);
   if (rc) return rc;
   B->bound = true;

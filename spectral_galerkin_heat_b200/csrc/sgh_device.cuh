@@ -269,7 +269,7 @@ __device__ __forceinline__ double laser_flux(const PP& P, double I0, double x0, 
   }
   const double ux = (x - x0) / P.r_x;
   const double uy = (y - y0) / P.r_y;
-  const double r2 = ux * ux + uy * uy;
+  const double r2 = __fma_rn(ux, ux, __dmul_rn(uy, uy));  // one rounding in every kernel this is compiled into
   const double shape = (P.order == 2.0) ? exp(-2.0 * r2) : exp(-2.0 * pow(r2, P.order / 2.0));
   return I0 * shape;
 }
