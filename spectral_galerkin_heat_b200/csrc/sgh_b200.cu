@@ -32,6 +32,7 @@
 #include "sgh_b200.h"
 #include "sgh_device.cuh"
 #include "sgh_fold.cuh"
+#include "sgh_volume.cuh"
 
 namespace {
 thread_local std::string g_last_error;
@@ -373,6 +374,12 @@ k_init_modes(const DevParams* __restrict__ P, const Ctrl* __restrict__ ctrl, dou
   a_it[i] = st_mode(t, P->round32);
 }
 
+// Committed modes of a mixed plan in the fused volume form: FP32 values.
+__global__ void __launch_bounds__(EW_THREADS) k_round_modes(double* a, int V) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < V) a[i] = st_mode(a[i], 1);
+}
+
 // a += KK w[p] S[y,x]  (add_bottom_surface_source, spectral_cpu_kernels.py:105-113)
 __global__ void __launch_bounds__(EW_THREADS)
 k_add_face(const DevParams* __restrict__ P, double* a, const double* __restrict__ KK,
@@ -461,8 +468,7 @@ k_stencil(const DevParams* __restrict__ P, const double* __restrict__ T, const d
   f[i] = dgx + dgy + dgz - a_prime(*P, t) * dTdt;
 }
 
-// Convergence test of one Picard iteration (solvers/spectral.py:464-499):
-// err = sqrt(sum res^2 / n) / max(sqrt(sum a_old^2 / n), 1e-9).
+// Sums of a relaxation's partials and the convergence test.
 __global__ void __launch_bounds__(EW_THREADS)
 k_converge(const DevParams* __restrict__ P, Ctrl* ctrl, const double* __restrict__ partials,
            int nparts, const double* __restrict__ extra_old, int n_extra,
@@ -476,29 +482,7 @@ k_converge(const DevParams* __restrict__ P, Ctrl* ctrl, const double* __restrict
   for (int b = threadIdx.x; b < n_extra; b += EW_THREADS) s1 += extra_old[b];
   block_sum2<EW_THREADS>(s0, s1, sh);
   if (threadIdx.x == 0) {
-    const double n = P->n_elements;
-    const double rms_d = sqrt(s0 / n);
-    const double rms_o = sqrt(s1 / n);
-    const double rel = rms_d / fmax(rms_o, 1e-9);
-    const int it = ctrl->iter + 1;
-    ctrl->iter = it;
-    ctrl->rel_err = rel;
-    if (ctrl->hist && it <= ctrl->hist_cap) {
-      ctrl->hist[2 * (it - 1)] = rms_d;
-      ctrl->hist[2 * (it - 1) + 1] = rel;
-    }
-    int stop = 0;
-    if (rel < P->tol) {
-      ctrl->status = SGH_STEP_CONVERGED;
-      stop = 1;
-    } else if (!isfinite(rel)) {
-      ctrl->status = SGH_STEP_NONFINITE;
-      stop = 1;
-    } else if (it >= P->max_iter) {
-      ctrl->status = SGH_STEP_CAPPED;
-      stop = 1;
-    }
-    ctrl->stop = stop;
+    const int stop = converge_test(*P, ctrl, s0, s1);
     if (in_graph) cudaGraphSetConditional(h_picard, stop ? 0u : 1u);
   }
 }
@@ -836,7 +820,10 @@ struct sgh_plan {
   // cluster form of the face-space step (cluster = 0: not used): packed folded
   // matrices (x forward, x inverse, y forward, y inverse) and volume partials
   int cluster = 0;
-  size_t o_fold[4] = {0, 0, 0, 0}, o_pv = 0;
+  // fused volume form (sgh_volume.cuh): CTAs per slab, 0: one pass per axis;
+  // o_fold[4..5]: packed z matrices
+  int slab = 0;
+  size_t o_fold[6] = {0, 0, 0, 0, 0, 0}, o_pv = 0;
   // box mode: point-major x/y tables, z reconstruction (+ face row) and
   // projection matrices, window bases, pass scratch, source and history
   double box_z0 = 0.0;
@@ -1207,6 +1194,10 @@ void enqueue_pre_begin(sgh_plan* p, cudaStream_t s, cudaGraphConditionalHandle h
   }
 }
 
+template <int MODE>
+void enqueue_slab(sgh_plan* p, const double* in, double* out, cudaStream_t s, cudaGraphConditionalHandle h_picard = 0,
+                  int in_graph = 0);
+
 // Rest of the step opening: (box mode) history shift and its projection,
 // initial guess and the convection guesses.
 void enqueue_pre_rest(sgh_plan* p, cudaStream_t s) {
@@ -1246,6 +1237,77 @@ void enqueue_pre_rest(sgh_plan* p, cudaStream_t s) {
                EpiConvFace{PP, h.h_bottom, h.prop_corr, p->d(p->o_f2), nullptr}, s);
     face_dct2(p, p->d(p->o_f2), p->d(p->o_Sbot), h.dct_scale, s);
   }
+  if (p->slab) enqueue_slab<vol::SLAB_INIT>(p, nullptr, p->d(p->o_t1), s);
+}
+
+// One slab kernel of the fused volume form (see sgh_volume.cuh).
+template <int MODE>
+void enqueue_slab(sgh_plan* p, const double* in, double* out, cudaStream_t s, cudaGraphConditionalHandle h_picard,
+                  int in_graph) {
+  const DevParams& h = p->hp;
+  const vol::SlabShape f = vol::slab_shape(h.nx, h.ny, p->slab);
+  vol::SlabArgs q = {};
+  q.P = point_phys(p->hp, p->P());
+  q.pxf = p->d(p->o_fold[0]); q.pxi = p->d(p->o_fold[1]);
+  q.pyf = p->d(p->o_fold[2]); q.pyi = p->d(p->o_fold[3]);
+  q.in = in;
+  q.qnet = p->d(p->o_qnet);
+  q.flux_scale = h.dct_scale / h.sqrt_dV;
+  q.aK = p->d(p->o_aK); q.KK = p->d(p->o_KK); q.Ct = p->d(p->o_ct); q.Cb = p->d(p->o_cb);
+  q.S_bot = h.has_bottom_conv ? p->d(p->o_Sbot) : nullptr;
+  q.a_trial = p->d(p->o_trial); q.a_it = p->d(p->o_a);
+  q.Qm = p->d(p->o_Qm);
+  q.out = out;
+  q.partials = p->d(p->o_prelax);
+  q.ctrl = p->ctrl();
+  q.h_picard = h_picard;
+  q.in_graph = in_graph;
+  if (f.keep)
+    SGH_CK_VOID(fold::launch_cluster(vol::k_slab<MODE, true>, f.n * h.nz, f.n, vol::SLAB_THREADS, f.bytes, true, s, f, q));
+  else
+    SGH_CK_VOID(fold::launch_cluster(vol::k_slab<MODE, false>, f.n * h.nz, f.n, vol::SLAB_THREADS, f.bytes, true, s, f, q));
+  ++g_launches;
+}
+
+// One column kernel of the fused volume form.
+template <int MODE>
+void enqueue_column(sgh_plan* p, const double* in, double* out, cudaStream_t s) {
+  const DevParams& h = p->hp;
+  const vol::ColShape f = vol::col_shape(h.nx, h.ny, h.nz);
+  vol::ColArgs q = {};
+  q.P = point_phys(p->hp, p->P());
+  q.pzf = p->d(p->o_fold[4]); q.pzi = p->d(p->o_fold[5]);
+  q.in = in;
+  q.Ct = p->d(p->o_ct);
+  q.inv_sqrt_dV = 1.0 / h.sqrt_dV;
+  q.latent = h.grid_latent;
+  q.rescale = h.prop_corr;
+  q.Tprev = p->d(p->o_Tprev);
+  q.q_las = p->d(p->o_qlas);
+  q.q_evap = p->d(p->o_qev); q.q_net = p->d(p->o_qnet);
+  q.out = out;
+  q.T = p->d(p->o_vol); q.kp = p->d(p->o_kp);
+  q.Tprev_out = p->d(p->o_Tprev); q.T_surf = p->d(p->o_Tsurf); q.q_evap_old = p->d(p->o_qevold);
+  q.partials = p->d(p->o_psurf);
+  (void)cudaFuncSetAttribute(vol::k_column<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, f.bytes);
+  launch_pdl(vol::k_column<MODE>, dim3(cdiv(h.S, f.cc)), vol::COL_THREADS, f.bytes, s, f, q);
+  ++g_launches;
+}
+
+// Picard iteration of the fused volume form; t1 holds the xy-inverse of the
+// iterate throughout, Qm the z-transformed latent source until the commit.
+void enqueue_picard_fused(sgh_plan* p, cudaStream_t s, cudaGraphConditionalHandle h_picard, int in_graph) {
+  const DevParams& h = p->hp;
+  double *B = p->d(p->o_t1), *C = p->d(p->o_t2), *G = p->d(p->o_Qm);
+  enqueue_column<vol::COL_LATENT>(p, B, G, s);
+  if (h.prop_corr) {
+    enqueue_slab<vol::SLAB_TRIAL>(p, h.grid_latent ? G : nullptr, C, s);
+    enqueue_column<vol::COL_TEMP>(p, C, nullptr, s);
+    enqueue_column<vol::COL_STENCIL>(p, nullptr, C, s);
+    enqueue_slab<vol::SLAB_RELAX>(p, C, B, s, h_picard, in_graph);
+  } else {
+    enqueue_slab<vol::SLAB_TRIAL_RELAX>(p, G, B, s, h_picard, in_graph);
+  }
 }
 
 void enqueue_pre(sgh_plan* p, cudaStream_t s) {
@@ -1257,6 +1319,10 @@ void enqueue_pre(sgh_plan* p, cudaStream_t s) {
 void enqueue_picard(sgh_plan* p, cudaStream_t s, cudaGraphConditionalHandle h_picard, int in_graph) {
   if (p->face_space) {
     enqueue_picard_face_space(p, s, h_picard, in_graph);
+    return;
+  }
+  if (p->slab) {
+    enqueue_picard_fused(p, s, h_picard, in_graph);
     return;
   }
   const DevParams& h = p->hp;
@@ -1380,6 +1446,14 @@ void enqueue_post(sgh_plan* p, cudaStream_t s, cudaGraphConditionalHandle h_step
         p->d(p->o_beta));
     ++g_launches;
     n_surf = p->nparts_surf;
+  } else if (p->slab) {
+    enqueue_column<vol::COL_COMMIT>(p, p->d(p->o_t1), nullptr, s);
+    n_surf = cdiv(h.S, vol::col_shape(h.nx, h.ny, h.nz).cc);
+    if (h.grid_latent) enqueue_slab<vol::SLAB_QM>(p, p->d(p->o_Qm), nullptr, s);
+    if (h.round32) {
+      k_round_modes<<<cdiv(h.V, EW_THREADS), EW_THREADS, 0, s>>>(p->d(p->o_a), h.V);
+      ++g_launches;
+    }
   } else if (h.grid_latent || h.prop_corr) {
     // T_prev and the surface temperature from one IDCT3 with the surface row
     volume_pass3(p, p->d(p->o_a), true,
@@ -1395,6 +1469,31 @@ void enqueue_post(sgh_plan* p, cudaStream_t s, cudaGraphConditionalHandle h_step
   k_commit<<<1, EW_THREADS, 0, s>>>(P, p->ctrl(), p->d(p->o_plas), p->nparts_las, p->d(p->o_psurf),
                                      n_surf, h_steps, in_graph);
   ++g_launches;
+}
+
+// Whether a property has distinct solid and liquid branches.
+bool phase_branches(const sgh_config& c) {
+  return std::memcmp(&c.k_solid, &c.k_liquid, sizeof(sgh_program)) != 0 ||
+         std::memcmp(&c.rho_solid, &c.rho_liquid, sizeof(sgh_program)) != 0 ||
+         std::memcmp(&c.c_solid, &c.c_liquid, sizeof(sgh_program)) != 0;
+}
+
+// CTAs per slab of the fused volume form, or 0 for one pass per axis: grid
+// mode in FP64, or in mixed precision (FP64 contractions there are more exact
+// than the split-BF16 ones and, fused, faster: 128 x 64 x 32, 3 steps, 14.3 -> 7.7
+// ms). One pass per axis remains for slabs that fit no cluster, for FP32 plans,
+// and for properties that jump between the phases: their fixed-point map need
+// not contract in grid mode (a 75 x 45 x 37 example runs to its cap of 80 in one
+// start of three), and rounding then grows to 1e-4 of the field within four
+// steps, so those plans keep the order of their sums (the fused form took 3.5
+// ms for that example's four steps, one pass per axis 6.8).
+int fused_slab(const sgh_plan* p) {
+  const DevParams& h = p->hp;
+  if (h.box || p->face_space || !(h.grid_latent || h.prop_corr)) return 0;
+  if (p->cfg.precision == SGH_PRECISION_FP32 || p->cfg.axis_cuda_cores) return 0;
+  if (h.prop_corr && phase_branches(p->cfg)) return 0;
+  if (vol::col_shape(h.nx, h.ny, h.nz).bytes > 200 * 1024) return 0;
+  return vol::slab_cluster(h.nx, h.ny, h.nz);
 }
 
 // Cluster size of the face-space step, or 0 for the multi-kernel form
@@ -1703,9 +1802,15 @@ int sgh_plan_create(const sgh_config* cfg, sgh_plan** out) {
   p->o_Ab = L.take(S8);
   p->o_pn1 = L.take(sizeof(double) * p->nparts_n1);
   p->cluster = face_cluster(p);
-  if (p->cluster) {
-    for (int q = 0; q < 4; ++q) p->o_fold[q] = L.take(sizeof(double) * fold::pack_doubles(q < 2 ? h.nx : h.ny));
-    p->o_pv = L.take(sizeof(double) * cdiv(h.S, FV_COLS));
+  p->slab = fused_slab(p);
+  if (p->cluster || p->slab) {
+    const int len[3] = {h.nx, h.ny, h.nz};
+    for (int q = 0; q < (p->slab ? 6 : 4); ++q) p->o_fold[q] = L.take(sizeof(double) * fold::pack_doubles(len[q / 2]));
+  }
+  if (p->cluster) p->o_pv = L.take(sizeof(double) * cdiv(h.S, FV_COLS));
+  if (p->slab) {
+    p->o_prelax = L.take(sizeof(double) * 2 * p->slab * h.nz);
+    p->o_psurf = L.take(sizeof(double) * 2 * cdiv(h.S, vol::col_shape(h.nx, h.ny, h.nz).cc));
   }
   if (c.precision == SGH_PRECISION_MIXED) {
     // each matrix with the largest (rows, contraction length) its passes use
@@ -1786,12 +1891,10 @@ int sgh_plan_bind(sgh_plan* p, void* workspace, uint64_t bytes, void* stream) {
     SGH_CK(cudaMemcpyAsync(p->d(p->o_bzi) + (size_t)h.zb * h.nz, p->d(p->o_ct), sizeof(double) * h.nz,
                            cudaMemcpyDeviceToDevice, s));
   }
-  if (p->cluster)
-    for (int q = 0; q < 2; ++q) {
-      const int N = q ? h.ny : h.nx;
-      fold::k_fold_pack<<<std::min(cdiv((long)fold::pack_doubles(N), EW_THREADS), 1184), EW_THREADS, 0, s>>>(
-          N, p->d(q ? p->o_my : p->o_mx), p->d(p->o_fold[2 * q]), p->d(p->o_fold[2 * q + 1]));
-    }
+  if (p->cluster || p->slab)
+    for (int q = 0; q < (p->slab ? 3 : 2); ++q)
+      fold::k_fold_pack<<<std::min(cdiv((long)fold::pack_doubles(mats[q].n), EW_THREADS), 1184), EW_THREADS, 0, s>>>(
+          mats[q].n, p->d(mats[q].m), p->d(p->o_fold[2 * q]), p->d(p->o_fold[2 * q + 1]));
   if (p->face_space)
     k_fs_weights<<<cdiv(h.S, EW_THREADS), EW_THREADS, 0, s>>>(p->P(), p->d(p->o_KK), p->d(p->o_ct),
                                                               p->d(p->o_cb), p->d(p->o_fsW));

@@ -62,6 +62,7 @@ struct Ctrl {
   // residual) per iteration, the first hist_cap iterations
   double* hist;
   int hist_cap;
+  unsigned tickets;  // CTAs of the current relaxation done (back to 0 after it)
   int umma_err;  // a split-BF16 tensor-core wait ran out (mixed-precision plans)
 };
 
@@ -356,6 +357,34 @@ __device__ __forceinline__ void block_max_sum(double& m, double& s, double* sh) 
       s += __shfl_down_sync(0xffffffffu, s, o);
     }
   }
+}
+
+// Convergence test of one Picard iteration (solvers/spectral.py:464-499):
+// err = sqrt(sum res^2 / n) / max(sqrt(sum a_old^2 / n), 1e-9). Updates the
+// control block; nonzero when the loop stops.
+__device__ __forceinline__ int converge_test(const DevParams& P, Ctrl* ctrl, double s0, double s1) {
+  const double rms_d = sqrt(s0 / P.n_elements);
+  const double rel = rms_d / fmax(sqrt(s1 / P.n_elements), 1e-9);
+  const int it = ctrl->iter + 1;
+  ctrl->iter = it;
+  ctrl->rel_err = rel;
+  if (ctrl->hist && it <= ctrl->hist_cap) {
+    ctrl->hist[2 * (it - 1)] = rms_d;
+    ctrl->hist[2 * (it - 1) + 1] = rel;
+  }
+  int stop = 0;
+  if (rel < P.tol) {
+    ctrl->status = SGH_STEP_CONVERGED;
+    stop = 1;
+  } else if (!isfinite(rel)) {
+    ctrl->status = SGH_STEP_NONFINITE;
+    stop = 1;
+  } else if (it >= P.max_iter) {
+    ctrl->status = SGH_STEP_CAPPED;
+    stop = 1;
+  }
+  ctrl->stop = stop;
+  return stop;
 }
 
 // Error reporting shared by the library's translation units (sgh_last_error).
