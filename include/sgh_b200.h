@@ -461,6 +461,11 @@ int sgh_nodal_workspace_bytes(int32_t nx, int32_t ny, int32_t nz, uint64_t* byte
 int sgh_nodal_temperature(int32_t nx, int32_t ny, int32_t nz, double Lx, double Ly, double Lz,
                           const double* modes, double* out, void* workspace, uint64_t bytes, void* stream);
 
+/* The same field in the reference's own axis order: out is C-ordered
+ * (nx+1, ny+1, nz+1), as reconstruct_temperature_DCT returns it. */
+int sgh_nodal_temperature_xyz(int32_t nx, int32_t ny, int32_t nz, double Lx, double Ly, double Lz,
+                              const double* modes, double* out, void* workspace, uint64_t bytes, void* stream);
+
 /* Temperature of FP64 modes at n_points points coords[3 i + 0..2] = (x, y, z),
  * each clipped to the domain: out[i] = sum a[p][n][m] C_m cos(pi m x / Lx)
  * C_n cos(pi n y / Ly) C_p cos(pi p z / Lz). Replaces

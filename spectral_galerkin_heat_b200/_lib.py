@@ -39,7 +39,7 @@ EXPORTED = (
     "sgh_plan_workspace_bytes", "sgh_plan_bind", "sgh_plan_buffer", "sgh_plan_launch_counts", "sgh_state_reset",
     "sgh_step", "sgh_step_eager", "sgh_run", "sgh_dct3d", "sgh_surface_temperature", "sgh_project_volume",
     "sgh_reconstruct_volume", "sgh_dctn_workspace_bytes", "sgh_dctn", "sgh_dctn_noalloc",
-    "sgh_nodal_workspace_bytes", "sgh_nodal_temperature", "sgh_points_workspace_bytes",
+    "sgh_nodal_workspace_bytes", "sgh_nodal_temperature", "sgh_nodal_temperature_xyz", "sgh_points_workspace_bytes",
     "sgh_points_temperature", "sgh_box_geometry", "sgh_box_window", "sgh_box_temperature",
     "sgh_box_project", "sgh_state_flags", "sgh_state_set_flags", "sgh_line_workspace_bytes",
     "sgh_line_temperature", "sgh_picard_history",
@@ -151,6 +151,8 @@ def lib() -> C.CDLL:
             "sgh_nodal_workspace_bytes": ([i32, i32, i32, u64p], C.c_int),
             "sgh_nodal_temperature": ([i32, i32, i32, C.c_double, C.c_double, C.c_double, vp, vp, vp,
                                        C.c_uint64, vp], C.c_int),
+            "sgh_nodal_temperature_xyz": ([i32, i32, i32, C.c_double, C.c_double, C.c_double, vp, vp, vp,
+                                           C.c_uint64, vp], C.c_int),
             "sgh_points_workspace_bytes": ([i32, i32, i32, i32, u64p], C.c_int),
             "sgh_points_temperature": ([i32, i32, i32, C.c_double, C.c_double, C.c_double, vp, i32, vp, vp,
                                         vp, C.c_uint64, vp], C.c_int),

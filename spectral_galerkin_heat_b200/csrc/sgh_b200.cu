@@ -32,6 +32,7 @@
 #include "sgh_b200.h"
 #include "sgh_device.cuh"
 #include "sgh_fold.cuh"
+#include "sgh_sym.cuh"
 #include "sgh_volume.cuh"
 
 namespace {
@@ -84,6 +85,23 @@ __global__ void k_dct_matrix(int N, double* M, double* MT) {
   const double v = w * cospi((double)m / (double)(2 * N));
   M[k * N + n] = v;
   MT[n * N + k] = v;
+}
+
+// The same for up to three axes at once (blockIdx.y = axis), only the matrix of
+// the direction asked for: M itself (inv = 0) or its transpose (inv = 1).
+struct DctAxes {
+  int n[3];
+  double* m[3];
+};
+__global__ void k_dct_axes(DctAxes q, int inv) {
+  const int N = q.n[blockIdx.y];
+  double* M = q.m[blockIdx.y];
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < (long long)N * N;
+       e += (long long)gridDim.x * blockDim.x) {
+    const int r = (int)(e / N), c = (int)(e - (long long)r * N), k = inv ? c : r, n = inv ? r : c;
+    const long long m = ((long long)k * (2 * n + 1)) % (4LL * N);
+    M[e] = ((k == 0) ? sqrt(1.0 / N) : sqrt(2.0 / N)) * cospi((double)m / (double)(2 * N));
+  }
 }
 
 // Propagators exactly as precompute_K_KK (physics/spectral_state.py:374-421):
@@ -2183,6 +2201,16 @@ int sgh_box_project(sgh_plan* p, const double* field_box, double* modes, void* s
 }
 
 namespace {
+// Whether a pass of sgh_dctn takes the halved contraction (sgh_sym.cuh): axes
+// below one tile, and long axes of few columns (under 40 of its CTAs), stay on
+// the small tiles of launch_axis. A pair of transforms, both ways measured: 96 x
+// 60 x 100 86 -> 66 us, 50 x 100 x 200 168 -> 117, 100 x 128 x 256 312 -> 250, 1-D
+// 1000 97 -> 90; 256 x 512, with 32 CTAs in its x-pass, 77 -> 80 halved.
+bool sym_pass(int N, long ncol) {
+  const long ctas = ((ncol + sym::BC - 1) / sym::BC) * (((N + 1) / 2 + sym::BJ - 1) / sym::BJ);
+  return N >= 16 && (ctas >= 40 || N <= 128 || ncol == 1);
+}
+
 struct DctnLayout {
   int n[3] = {1, 1, 1};   // (n0, n1, n2), n2 fastest; unused leading axes are 1
   int ndim = 0;
@@ -2229,13 +2257,15 @@ int sgh_dctn(int32_t kind, int32_t ndim, const int32_t* shape, const double* in,
     return fail(SGH_ERR_WORKSPACE, "workspace must be 256-byte aligned");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   char* ws = static_cast<char*>(workspace);
-  const double* mats[3];
-  for (int a = 0; a < 3; ++a) {
-    const int N = L.n[a];
-    double* M = reinterpret_cast<double*>(ws + L.o_mat[a]);
-    k_dct_matrix<<<cdiv((long)N * N, EW_THREADS), EW_THREADS, 0, s>>>(N, M, M + (size_t)N * N);
-    mats[a] = (kind == 2) ? M : M + (size_t)N * N;
+  DctAxes ax;
+  int longest = 1;
+  for (int a = 0; a < L.ndim; ++a) {
+    ax.n[a] = L.n[3 - L.ndim + a];
+    ax.m[a] = reinterpret_cast<double*>(ws + L.o_mat[3 - L.ndim + a]);
+    longest = std::max(longest, ax.n[a]);
   }
+  k_dct_axes<<<dim3(std::min(cdiv((long)longest * longest, EW_THREADS), 592), L.ndim), EW_THREADS, 0, s>>>(
+      ax, kind == 2 ? 0 : 1);
   double* t1 = reinterpret_cast<double*>(ws + L.o_t1);
   double* t2 = reinterpret_cast<double*>(ws + L.o_t2);
   const int n0 = L.n[0], n1 = L.n[1], n2 = L.n[2];
@@ -2253,7 +2283,11 @@ int sgh_dctn(int32_t kind, int32_t ndim, const int32_t* shape, const double* in,
     const int N = L.n[a];
     const int A = (a == 2) ? n0 * n1 : (a == 1 ? n0 : 1);
     const int B = (a == 2) ? 1 : (a == 1 ? n2 : n1 * n2);
-    launch_axis(src, mats[a], N, N, A, B, EpiStore{dst, 1.0, nullptr}, s);
+    const double* M = reinterpret_cast<const double*>(ws + L.o_mat[a]);
+    if (sym_pass(N, (long)A * B))
+      sym::launch(kind, src, M, dst, N, N, A, B, (long long)N * B, B, B == 1, s);
+    else
+      launch_axis(src, M, N, N, A, B, EpiStore{dst, 1.0, nullptr}, s);
     src = dst;
   }
   SGH_CK(cudaGetLastError());

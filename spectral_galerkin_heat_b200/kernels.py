@@ -12,7 +12,7 @@ Functions with the reference kernel modules' names and meanings
   ``sgh_project_volume``;
 * output reconstruction with the reference's names and arguments
   (``physics/spectral_helpers.py``): ``reconstruct_temperature_DCT(a, state)``
-  (node-centred field, :146-204) -> ``sgh_nodal_temperature``;
+  (node-centred field, :146-204) -> ``sgh_nodal_temperature_xyz``;
   ``reconstruct_temperature_volume_at_points(a, num, geom, state, coords)``
   (:206-248) -> ``sgh_points_temperature``; ``save_temp_profiles(a, num, geom,
   state, laser_position, center, num_points)`` (:251-333), each line reduced
@@ -185,11 +185,11 @@ def reconstruct_temperature_DCT(a, state):
     nbytes = C.c_uint64()
     _lib.check("sgh_nodal_workspace_bytes", L.sgh_nodal_workspace_bytes(nx, ny, nz, C.byref(nbytes)))
     ws = _workspace("nodal", nbytes.value, a.device)
-    out = torch.empty((nz + 1, ny + 1, nx + 1), dtype=torch.float64, device=a.device)
-    _lib.check("sgh_nodal_temperature", L.sgh_nodal_temperature(
+    out = torch.empty((nx + 1, ny + 1, nz + 1), dtype=torch.float64, device=a.device)
+    _lib.check("sgh_nodal_temperature_xyz", L.sgh_nodal_temperature_xyz(
         nx, ny, nz, Lx, Ly, Lz, C.c_void_p(a.data_ptr()), C.c_void_p(out.data_ptr()),
         C.c_void_p(ws.data_ptr()), ws.numel(), C.c_void_p(torch.cuda.current_stream(a.device).cuda_stream)))
-    return out.permute(2, 1, 0).contiguous()
+    return out
 
 
 def reconstruct_temperature_volume_at_points(a, num, geom, state, coords):
