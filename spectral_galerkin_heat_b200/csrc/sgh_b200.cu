@@ -505,10 +505,12 @@ k_converge(const DevParams* __restrict__ P, Ctrl* ctrl, const double* __restrict
   }
 }
 
-// Where k_converge records the Picard history of a step.
-__global__ void k_ctrl_history(Ctrl* ctrl, double* hist, int cap) {
+// Where the convergence test records the Picard history of a step, and where a
+// single step writes its metrics for the host.
+__global__ void k_ctrl_setup(Ctrl* ctrl, double* hist, int cap, sgh_step_out* host_out) {
   ctrl->hist = hist;
   ctrl->hist_cap = cap;
+  ctrl->host_out = host_out;
 }
 
 // Metrics and history of the committed step (solvers/spectral.py:502-542);
@@ -547,6 +549,7 @@ k_commit(const DevParams* __restrict__ P, Ctrl* ctrl, const double* __restrict__
     o.flags = flags;
     ctrl->out = o;
     if (ctrl->out_table) ctrl->out_table[ctrl->step] = o;
+    else *ctrl->host_out = o;
     if (P->grid_latent && P->max_iter > 0) ctrl->have_qprev = 1;
     const int next = ctrl->step + 1;
     ctrl->step = next;
@@ -800,6 +803,7 @@ k_face_run(const DevParams* __restrict__ P, Ctrl* ctrl, fold::FaceShape f, fold:
     ctrl->rel_err = r.rel;
     ctrl->out = o;
     if (ctrl->out_table) ctrl->out_table[step] = o;
+    else *ctrl->host_out = o;
     ctrl->step = step + 1;
     if (in_graph) cudaGraphSetConditional(h_steps, step + 1 < ctrl->n_target ? 1u : 0u);
   }
@@ -860,6 +864,10 @@ struct sgh_plan {
   bool bound_planes = false;
   size_t ws_need = 0;
   char* ws = nullptr;
+  // Metrics of a single step, pinned: the step's last kernel writes them, so that
+  // sgh_step needs no device-to-host copy before it waits (eight steps of a 64 x
+  // 32 x 16 track: 398 us with a copy to pageable memory, 346 without).
+  sgh_step_out* host_out = nullptr;
   bool bound = false;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -1861,6 +1869,7 @@ int sgh_plan_destroy(sgh_plan* p) {
   if (p->graph) cudaGraphDestroy(p->graph);
   if (p->cs1) cudaStreamDestroy(p->cs1);
   if (p->cs2) cudaStreamDestroy(p->cs2);
+  if (p->host_out) cudaFreeHost(p->host_out);
   delete p;
   return SGH_OK;
 }
@@ -1885,7 +1894,11 @@ int sgh_plan_bind(sgh_plan* p, void* workspace, uint64_t bytes, void* stream) {
   const DevParams& h = p->hp;
   SGH_CK(cudaMemcpyAsync(p->P(), &h, sizeof(DevParams), cudaMemcpyHostToDevice, s));
   SGH_CK(cudaMemsetAsync(p->ctrl(), 0, sizeof(Ctrl), s));
-  k_ctrl_history<<<1, 1, 0, s>>>(p->ctrl(), p->d(p->o_hist), p->hist_cap);
+  if (!p->host_out)
+    SGH_CK(cudaHostAlloc(&p->host_out, sizeof(sgh_step_out), cudaHostAllocMapped | cudaHostAllocPortable));
+  sgh_step_out* host_out_dev = nullptr;
+  SGH_CK(cudaHostGetDevicePointer(&host_out_dev, p->host_out, 0));
+  k_ctrl_setup<<<1, 1, 0, s>>>(p->ctrl(), p->d(p->o_hist), p->hist_cap, host_out_dev);
   struct { int n; size_t m, mt; } mats[3] = {{h.nx, p->o_mx, p->o_mxt}, {h.ny, p->o_my, p->o_myt},
                                              {h.nz, p->o_mz, p->o_mzt}};
   for (auto& m : mats)
@@ -2015,15 +2028,15 @@ int sgh_step(sgh_plan* p, const sgh_laser* laser, sgh_step_out* out, void* strea
     enqueue_face_run(p, s, 0, 0);
     enqueue_fs_volume<true, false>(p, s, sgh_laser{}, nullptr, nullptr, 0);
     SGH_CK(cudaGetLastError());
-    if (out) SGH_CK(cudaMemcpyAsync(out, &p->ctrl()->out, sizeof(sgh_step_out), cudaMemcpyDeviceToHost, s));
     SGH_CK(cudaStreamSynchronize(s));
+    if (out) *out = *p->host_out;
     return SGH_OK;
   }
   k_run_setup<<<1, 1, 0, s>>>(p->ctrl(), *laser, nullptr, nullptr, 1);
   SGH_CK(cudaGetLastError());
   SGH_CK(cudaGraphLaunch(p->exec, s));
-  if (out) SGH_CK(cudaMemcpyAsync(out, &p->ctrl()->out, sizeof(sgh_step_out), cudaMemcpyDeviceToHost, s));
   SGH_CK(cudaStreamSynchronize(s));
+  if (out) *out = *p->host_out;
   return SGH_OK;
 }
 
@@ -2045,8 +2058,8 @@ int sgh_step_eager(sgh_plan* p, const sgh_laser* laser, sgh_step_out* out, void*
   }
   enqueue_post(p, s, 0, 0);
   SGH_CK(cudaGetLastError());
-  if (out) SGH_CK(cudaMemcpyAsync(out, &p->ctrl()->out, sizeof(sgh_step_out), cudaMemcpyDeviceToHost, s));
   SGH_CK(cudaStreamSynchronize(s));
+  if (out) *out = *p->host_out;
   return SGH_OK;
 }
 

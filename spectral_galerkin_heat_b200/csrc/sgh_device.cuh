@@ -51,6 +51,7 @@ struct Ctrl {
   double I0, shift_x, shift_y;  // peak intensity and warm-start shift (pixels)
   double rel_err;
   sgh_step_out out;         // metrics of the last step
+  sgh_step_out* host_out;   // where a single step's metrics go (pinned host memory)
   // box mode: history present (FineMeshState.T_prev is not None), window
   // start indices, history shift in fine pixels, and the magnitude maxima of
   // the committed latent source (peak, floor, x edges, y edges) as the bit
