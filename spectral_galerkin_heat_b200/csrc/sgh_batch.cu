@@ -277,17 +277,46 @@ __global__ void __launch_bounds__(BT) kb_weights(BView v, const R* KK, R* Wtt, R
   Qtt[sl.face + i] = (R)q;
 }
 
-// (Re)start one slot at the initial condition (solvers/spectral.py:176-180).
+// (Re)start one slot at the initial condition (solvers/spectral.py:176-180). Only
+// the zero mode is set, so the first step's face sums and norm are one term
+// each: they are written here, with the volume pass's arithmetic, instead of
+// read from the whole volume before the first step (48 serving slots started
+// and stepped five times: 1441 -> 1386 us). Four modes per thread.
 template <class R>
 __global__ void __launch_bounds__(BT)
-kb_slot_start(BView v, int s, R* a, double* q_evold, double* sigma, const sgh_laser* table,
-              int n_steps, sgh_step_out* outs) {
+kb_slot_start(BView v, int s, R* a, const R* K, const R* KK, double* q_evold, double* sigma, R* Zt, R* Yt,
+              double* part_n1, const sgh_laser* table, int n_steps, sgh_step_out* outs) {
+  constexpr bool TAB = sizeof(R) == 4;
   const BSlot& sl = v.slot[s];
   const long long i = (long long)blockIdx.x * BT + threadIdx.x;
-  if (i < sl.V) a[sl.vol + i] = (R)((i == 0) ? sl.T0 * sqrt(sl.Lx * sl.Ly * sl.Lz) : 0.0);
+  const R a0 = (R)(sl.T0 * sqrt(sl.Lx * sl.Ly * sl.Lz));
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    if (4 * i + c < sl.V) a[sl.vol + 4 * i + c] = 4 * i + c == 0 ? a0 : (R)0;
   if (i < sl.S) {
     q_evold[sl.face + i] = 0.0;
     sigma[sl.face + i] = 0.0;
+    R z = (R)0, y = (R)0;
+    double n1 = 0.0;
+    if (i == 0) {
+      if (TAB) {
+        const double* E = v.E + sl.eoff;
+        const float kv = (float)(E[0] * E[sl.nx]) * (float)E[sl.nx + sl.ny], cp = (float)v.Ct[sl.zoff];
+        const float t = (float)(sl.dt / (sl.rho * sl.cp)) * cp, ak = (float)a0 * kv;
+        z = (R)fmaf(cp, ak, 0.0f);
+        y = (R)fmaf(ak, t, 0.0f);
+        n1 = (double)fmaf(ak, ak, 0.0f);
+      } else {
+        const double kv = (double)K[sl.vol], kk = (double)KK[sl.vol], cp = v.Ct[sl.zoff];
+        const double ak = __dmul_rn((double)a0, kv);
+        z = (R)fma(cp, ak, 0.0);
+        y = (R)fma(ak * kk, cp, 0.0);
+        n1 = fma(ak, ak, 0.0);
+      }
+    }
+    Zt[sl.face + i] = z;
+    Yt[sl.face + i] = y;
+    if (i < sl.nblk) part_n1[sl.blk0 + i] = n1;
   }
   if (i == 0) {
     BState& st = v.st[s];
@@ -299,7 +328,7 @@ kb_slot_start(BView v, int s, R* a, double* q_evold, double* sigma, const sgh_la
     st.iters = 0;
     st.done = 1;
     st.iter = 0;
-    st.pass1_ready = 0;
+    st.pass1_ready = 1;
   }
 }
 
@@ -2262,14 +2291,15 @@ int sgh_batch_slot_start(sgh_batch* B, int32_t slot, const sgh_laser* lasers_dev
   if (n_steps < 0 || (n_steps > 0 && !lasers_dev)) return bfail(SGH_ERR_INVALID, "bad laser table");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const BSlot& sl = B->slots[slot];
-  const int g = cdivl(std::max<long long>(sl.V, sl.S), BT);
+  const int g = cdivl(std::max<long long>((sl.V + 3) / 4, sl.S), BT);
   if (B->precision == SGH_PRECISION_MIXED)
-    kb_slot_start<float><<<g, BT, 0, s>>>(B->view(), slot, reinterpret_cast<float*>(B->ws + B->o_a),
-                                          B->d(B->o_qevold), B->d(B->o_sigma), lasers_dev,
-                                          n_steps, outs_dev);
+    kb_slot_start<float><<<g, BT, 0, s>>>(B->view(), slot, B->f(B->o_a), nullptr, nullptr, B->d(B->o_qevold),
+                                          B->d(B->o_sigma), B->f(B->o_Zt), B->f(B->o_Yt), B->d(B->o_pn1),
+                                          lasers_dev, n_steps, outs_dev);
   else
-    kb_slot_start<double><<<g, BT, 0, s>>>(B->view(), slot, B->d(B->o_a), B->d(B->o_qevold), B->d(B->o_sigma),
-                                           lasers_dev, n_steps, outs_dev);
+    kb_slot_start<double><<<g, BT, 0, s>>>(B->view(), slot, B->d(B->o_a), B->d(B->o_K), B->d(B->o_KK),
+                                           B->d(B->o_qevold), B->d(B->o_sigma), B->d(B->o_Zt), B->d(B->o_Yt),
+                                           B->d(B->o_pn1), lasers_dev, n_steps, outs_dev);
   SGB_CK(cudaGetLastError());
   return SGH_OK;
 }
