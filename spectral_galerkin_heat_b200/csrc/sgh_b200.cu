@@ -768,6 +768,7 @@ k_fs_volume(Ctrl* ctrl, sgh_laser laser, const sgh_laser* table, sgh_step_out* o
 
 // Step opening, Picard loop, surface commit and metrics of one instance in one
 // cluster (solvers/spectral.py:258-268, 273-306, 386-512, 536-542).
+template <bool KEEPM>
 __global__ void __launch_bounds__(fold::FACE_THREADS, 1)
 k_face_run(const DevParams* __restrict__ P, Ctrl* ctrl, fold::FaceShape f, fold::FaceJob<double> J,
            cudaGraphConditionalHandle h_steps, int in_graph) {
@@ -783,7 +784,7 @@ k_face_run(const DevParams* __restrict__ P, Ctrl* ctrl, fold::FaceShape f, fold:
   J.shift_x = laser_shift(L.vx, P->dt, P->dx, f32);
   J.shift_y = laser_shift(L.vy, P->dt, P->dy, f32);
   const bool ok = fold::face_operands(f, J, fr_sh, bar, umma::WAIT_LIMIT, false, &ctrl->umma_err);
-  const fold::FaceResult r = fold::face_step(f, J, fr_sh, !ok);
+  const fold::FaceResult r = fold::face_step<double, KEEPM>(f, J, fr_sh, !ok);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     sgh_step_out o;
     o.T_surface_max = r.tmax;
@@ -1182,8 +1183,12 @@ void enqueue_fs_volume(sgh_plan* p, cudaStream_t s, const sgh_laser& laser, cons
 }
 void enqueue_face_run(sgh_plan* p, cudaStream_t s, cudaGraphConditionalHandle h_steps, int in_graph) {
   const fold::FaceShape f = fold::face_shape<double>(p->hp.nx, p->hp.ny, p->cluster);
-  SGH_CK_VOID(fold::launch_cluster(k_face_run, f.n, f.n, fold::threads_for(f), f.bytes, true, s, p->P(), p->ctrl(), f, face_job(p), h_steps,
-                                   in_graph));
+  auto go = [&](auto kernel) {
+    SGH_CK_VOID(fold::launch_cluster(kernel, f.n, f.n, fold::threads_for(f), f.bytes, true, s, p->P(), p->ctrl(), f,
+                                     face_job(p), h_steps, in_graph));
+  };
+  if (f.keep & fold::FACE_M) go(k_face_run<true>);
+  else go(k_face_run<false>);
   ++g_launches;
 }
 

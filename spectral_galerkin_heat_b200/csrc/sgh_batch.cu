@@ -1204,7 +1204,7 @@ struct FaceArrays {
   double *qlas, *qev, *sigma, *Tsurf;
   const double* fold;
 };
-template <class W>
+template <class W, bool KEEPM>
 __global__ void __launch_bounds__(fold::FACE_THREADS, 1)
 kb_face_cluster(BView v, const int* list, const fold::FaceShape* shape, int cl, FaceArrays q) {
   extern __shared__ __align__(128) double fc_sh[];
@@ -1233,7 +1233,7 @@ kb_face_cluster(BView v, const int* list, const fold::FaceShape* shape, int cl, 
   J.hist_cap = 0;
   const unsigned lim = v.g->wait_limit ? v.g->wait_limit : umma::WAIT_LIMIT;
   const bool ok = fold::face_operands(f, J, fc_sh, bar, lim, v.g->stall_test != 0, &v.g->umma_err);
-  const fold::FaceResult r = fold::face_step(f, J, fc_sh, !ok);
+  const fold::FaceResult r = fold::face_step<W, KEEPM>(f, J, fc_sh, !ok);
   if (blockIdx.x % cl == 0 && threadIdx.x == 0) {
     st.iter = r.iter;
     st.status = r.status;
@@ -1640,10 +1640,11 @@ struct sgh_batch {
   // launch groups over clist, per-slot shapes, packed folded matrices
   struct ClusterGroup {
     int n, first, count, threads, bytes;
+    bool keepm;  // the packed matrices fit in the shared memory of every slot of the group
   };
   std::vector<ClusterGroup> cgroups;
-  cudaStream_t gs[5] = {};  // streams and events of the groups beyond the first
-  cudaEvent_t ge[5] = {};
+  cudaStream_t gs[10] = {};  // streams and events of the groups beyond the first
+  cudaEvent_t ge[10] = {};
   std::vector<int> clist;
   std::vector<fold::FaceShape> cshape;
   std::vector<std::pair<int, long long>> fold_list;  // (N, element offset: forward, inverse)
@@ -1774,9 +1775,13 @@ void enqueue_clusters(sgh_batch* B, cudaStream_t s) {
     cudaStream_t t = k ? B->gs[k] : s;
     if (k == 0 && ng > 1) (void)cudaEventRecord(B->ge[0], s);
     if (k) (void)cudaStreamWaitEvent(t, B->ge[0], 0);
-    (void)fold::launch_cluster(kb_face_cluster<R>, g.n * g.count, g.n, g.threads, g.bytes, false, t, B->view(),
-                               reinterpret_cast<const int*>(B->ws + B->o_clist) + g.first,
-                               reinterpret_cast<const fold::FaceShape*>(B->ws + B->o_cshape), g.n, q);
+    auto go = [&](auto kernel) {
+      (void)fold::launch_cluster(kernel, g.n * g.count, g.n, g.threads, g.bytes, false, t, B->view(),
+                                 reinterpret_cast<const int*>(B->ws + B->o_clist) + g.first,
+                                 reinterpret_cast<const fold::FaceShape*>(B->ws + B->o_cshape), g.n, q);
+    };
+    if (g.keepm) go(kb_face_cluster<R, true>);
+    else go(kb_face_cluster<R, false>);
     g_blaunch += 1;
     if (k) (void)cudaEventRecord(B->ge[k], t);
   }
@@ -2094,23 +2099,27 @@ int sgh_batch_create(const sgh_config* cfgs, int32_t n, int32_t precision, sgh_b
     }
   }
   B->cshape.resize(n);
-  for (int cl = fold::FACE_MAX_CLUSTER; cl >= 1; cl /= 2) {
-    sgh_batch::ClusterGroup g = {cl, (int)B->clist.size(), 0, 0, 0};
-    std::vector<int> m;
-    for (int i = 0; i < n; ++i)
-      if (B->slots[i].cl == cl) m.push_back(i);
-    std::stable_sort(m.begin(), m.end(), [&](int a, int b) { return B->slots[a].S > B->slots[b].S; });
-    for (int i : m) {
-      const BSlot& sl = B->slots[i];
-      B->cshape[i] = precision == SGH_PRECISION_MIXED ? fold::face_shape<float>(sl.nx, sl.ny, cl)
-                                                      : fold::face_shape<double>(sl.nx, sl.ny, cl);
-      g.threads = std::max(g.threads, fold::threads_for(B->cshape[i]));
-      g.bytes = std::max(g.bytes, B->cshape[i].bytes);
-    }
-    g.count = (int)m.size();
-    B->clist.insert(B->clist.end(), m.begin(), m.end());
-    if (g.count) B->cgroups.push_back(g);
+  for (int i = 0; i < n; ++i) {
+    const BSlot& sl = B->slots[i];
+    if (sl.cl)
+      B->cshape[i] = precision == SGH_PRECISION_MIXED ? fold::face_shape<float>(sl.nx, sl.ny, sl.cl)
+                                                      : fold::face_shape<double>(sl.nx, sl.ny, sl.cl);
   }
+  for (int cl = fold::FACE_MAX_CLUSTER; cl >= 1; cl /= 2)
+    for (int keepm = 0; keepm < 2; ++keepm) {
+      sgh_batch::ClusterGroup g = {cl, (int)B->clist.size(), 0, 0, 0, keepm != 0};
+      std::vector<int> m;
+      for (int i = 0; i < n; ++i)
+        if (B->slots[i].cl == cl && ((B->cshape[i].keep & fold::FACE_M) != 0) == g.keepm) m.push_back(i);
+      std::stable_sort(m.begin(), m.end(), [&](int a, int b) { return B->slots[a].S > B->slots[b].S; });
+      for (int i : m) {
+        g.threads = std::max(g.threads, fold::threads_for(B->cshape[i]));
+        g.bytes = std::max(g.bytes, B->cshape[i].bytes);
+      }
+      g.count = (int)m.size();
+      B->clist.insert(B->clist.end(), m.begin(), m.end());
+      if (g.count) B->cgroups.push_back(g);
+    }
   {
     const int vw = precision == SGH_PRECISION_MIXED ? 4 : 2;
     bool ok = true;
@@ -2176,7 +2185,7 @@ int sgh_batch_destroy(sgh_batch* B) {
   if (B->graph) cudaGraphDestroy(B->graph);
   if (B->cs1) cudaStreamDestroy(B->cs1);
   if (B->cs2) cudaStreamDestroy(B->cs2);
-  for (int k = 0; k < 5; ++k) {
+  for (int k = 0; k < 10; ++k) {
     if (B->gs[k]) cudaStreamDestroy(B->gs[k]);
     if (B->ge[k]) cudaEventDestroy(B->ge[k]);
   }

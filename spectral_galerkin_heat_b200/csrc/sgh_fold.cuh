@@ -323,8 +323,9 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 // All threads of all CTAs of the cluster. The result is complete on rank 0,
 // thread 0. bad: this CTA's operands are invalid (an expired wait): its
-// partials become NaN and the step ends non-finite.
-template <class W>
+// partials become NaN and the step ends non-finite. KEEPM: the packed matrices
+// are in shared memory (FACE_M), addressed as such.
+template <class W, bool KEEPM>
 __device__ FaceResult face_step(const FaceShape& f, const FaceJob<W>& J, double* sm, bool bad) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
@@ -349,14 +350,11 @@ __device__ FaceResult face_step(const FaceShape& f, const FaceJob<W>& J, double*
   W* sw = reinterpret_cast<W*>(sm + f.o_w);
   const int wstride = ny * ldc;
   double* sq = sm + f.o_q;
-  const double *pxf = J.pxf, *pxi = J.pxi, *pyf = J.pyf, *pyi = J.pyi;
-  if (f.keep & FACE_M) {
-    const size_t nxp = pack_doubles(nx), nyp = pack_doubles(ny);
-    pxf = sm + f.o_m;
-    pxi = pxf + nxp;
-    pyf = pxi + nxp;
-    pyi = pyf + nyp;
-  }
+  const int nxp = (int)pack_doubles(nx), nyp = (int)pack_doubles(ny);
+  const double* pxf = KEEPM ? sm + f.o_m : J.pxf;
+  const double* pxi = KEEPM ? sm + f.o_m + nxp : J.pxi;
+  const double* pyf = KEEPM ? sm + f.o_m + 2 * nxp : J.pyf;
+  const double* pyi = KEEPM ? sm + f.o_m + 2 * nxp + nyp : J.pyi;
 
   if (keepw) {  // this CTA's columns of the face sums and weights, in position order
     for (int p = warp; p < ny; p += NW) {
