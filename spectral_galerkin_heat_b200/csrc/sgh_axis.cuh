@@ -491,6 +491,9 @@ k_axis_mma(const double* __restrict__ X, const double* __restrict__ Mat, int Nou
 // while the previous kernel of the stream finishes, and must execute
 // griddepcontrol.wait before its first global access (every kernel launched
 // here does, in all CTAs).
+// Cleared around a launch that follows a join of streams (its dependencies are
+// not one kernel of its own stream).
+inline thread_local bool g_pdl = true;
 template <class... KArgs, class... Args>
 inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, int smem, cudaStream_t st,
                        Args&&... args) {
@@ -503,7 +506,7 @@ inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, int sme
   la[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   la[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = la;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = g_pdl ? 1 : 0;
   cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 

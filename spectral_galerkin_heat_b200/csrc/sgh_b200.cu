@@ -873,6 +873,8 @@ struct sgh_plan {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   cudaStream_t cs1 = nullptr, cs2 = nullptr;
+  cudaStream_t fs = nullptr;  // box mode: the top face beside the box passes
+  cudaEvent_t fe[2] = {};
 
   template <class T>
   T* at(size_t off) const { return reinterpret_cast<T*>(ws + off); }
@@ -1074,13 +1076,28 @@ void box_xy(sgh_plan* p, const Epi& epi, cudaStream_t s) {
 // Projection of a box field onto the modes (project_box_to_modes,
 // physics/spectral_ops.py:53-74); epi receives the contraction before the
 // dV_fine scale.
-template <class Epi>
-void box_project(sgh_plan* p, const double* field, const Epi& epi, cudaStream_t s) {
+void box_project_yx(sgh_plan* p, const double* field, cudaStream_t s) {
   const DevParams& h = p->hp;
   axis(field, p->d(p->o_wyf), h.ny, h.yb, h.zb, h.xb, EpiStore{p->d(p->o_bt2), 1.0, nullptr}, s);
   axis(p->d(p->o_bt2), p->d(p->o_wxf), h.nx, h.xb, h.zb * h.ny, 1, EpiStore{p->d(p->o_bt1), 1.0, nullptr}, s);
+}
+template <class Epi>
+void box_project_z(sgh_plan* p, const Epi& epi, cudaStream_t s) {
+  const DevParams& h = p->hp;
   axis(p->d(p->o_bt1), p->d(p->o_bzf), h.nz, h.zb, 1, h.S, epi, s);
 }
+template <class Epi>
+void box_project(sgh_plan* p, const double* field, const Epi& epi, cudaStream_t s) {
+  box_project_yx(p, field, s);
+  box_project_z(p, epi, s);
+}
+
+// Launches without programmatic serialisation while it lives.
+struct NoPdl {
+  bool saved = g_pdl;
+  NoPdl() { g_pdl = false; }
+  ~NoPdl() { g_pdl = saved; }
+};
 
 // First step of a run: seed T_prev = T_box(aK) and Q_prev = 0
 // (initialize_latent_heat_if_needed, physics/spectral_ops.py:182-194). Every
@@ -1367,24 +1384,39 @@ void enqueue_picard(sgh_plan* p, cudaStream_t s, cudaGraphConditionalHandle h_pi
     // box z-pass with the face row, top flux from the face row, the latent
     // source on the box, and its projection into the trial modes
     // (solvers/spectral.py:388-443 with the box branch :413-422)
+    // The top face's transforms (four launches of a 48 x 80 face) and the box's x
+    // and y passes both start from the z-pass and meet in the trial modes: the
+    // face runs beside the box on a forked stream. 80 x 48 x 120 with a 160 x 96 x
+    // 112 box, 4 steps: 11.5 -> 10.3 ms.
     box_zpass(p, p->d(p->o_a), true, s);
-    face_idct2_from(p, p->d(p->o_bt1) + (size_t)h.zb * h.S,
-                    EpiTopFlux{PP, p->d(p->o_qlas), p->d(p->o_qev), p->d(p->o_qnet), h.prop_corr, nullptr}, s);
-    face_dct2(p, p->d(p->o_qnet), p->d(p->o_Stop), h.dct_scale, s);
+    SGH_CK_VOID(cudaEventRecord(p->fe[0], s));
+    SGH_CK_VOID(cudaStreamWaitEvent(p->fs, p->fe[0], 0));
+    {
+      NoPdl first;
+      axis(p->d(p->o_bt1) + (size_t)h.zb * h.S, p->d(p->o_mxt), h.nx, h.nx, h.ny, 1,
+           EpiStore{p->d(p->o_f1), 1.0, nullptr}, p->fs);
+    }
+    axis(p->d(p->o_f1), p->d(p->o_myt), h.ny, h.ny, 1, h.nx,
+         EpiTopFlux{PP, p->d(p->o_qlas), p->d(p->o_qev), p->d(p->o_qnet), h.prop_corr, nullptr}, p->fs);
+    face_dct2(p, p->d(p->o_qnet), p->d(p->o_Stop), h.dct_scale, p->fs);
+    SGH_CK_VOID(cudaEventRecord(p->fe[1], p->fs));
     box_xy(p, EpiBoxLatent{PP, p->d(p->o_Tsh), p->d(p->o_Qbox), nullptr, h.latent_model, h.T_solidus, h.band_inv,
                            h.latent_factor},
            s);
+    box_project_yx(p, p->d(p->o_Qbox), s);
+    SGH_CK_VOID(cudaStreamWaitEvent(s, p->fe[1], 0));
+    NoPdl joined;
     if (h.prop_corr) {
-      box_project(p, p->d(p->o_Qbox),
-                  EpiTrial<false>{PP, p->d(p->o_aK), p->d(p->o_KK), p->d(p->o_ct), p->d(p->o_cb), p->d(p->o_Stop),
-                                  1.0, h.dV_fine, S_bot, nullptr, p->d(p->o_trial), nullptr, nullptr, h.S, h.omega},
-                  s);
+      box_project_z(p,
+                    EpiTrial<false>{PP, p->d(p->o_aK), p->d(p->o_KK), p->d(p->o_ct), p->d(p->o_cb), p->d(p->o_Stop),
+                                    1.0, h.dV_fine, S_bot, nullptr, p->d(p->o_trial), nullptr, nullptr, h.S, h.omega},
+                    s);
     } else {
-      box_project(p, p->d(p->o_Qbox),
-                  EpiTrial<true>{PP, p->d(p->o_aK), p->d(p->o_KK), p->d(p->o_ct), p->d(p->o_cb), p->d(p->o_Stop),
-                                 1.0, h.dV_fine, S_bot, nullptr, nullptr, p->d(p->o_a), p->d(p->o_prelax), h.S,
-                                 h.omega},
-                  s);
+      box_project_z(p,
+                    EpiTrial<true>{PP, p->d(p->o_aK), p->d(p->o_KK), p->d(p->o_ct), p->d(p->o_cb), p->d(p->o_Stop),
+                                   1.0, h.dV_fine, S_bot, nullptr, nullptr, p->d(p->o_a), p->d(p->o_prelax), h.S,
+                                   h.omega},
+                    s);
       nparts = axis_blocks(h.nz, 1, h.S);
     }
   } else if (h.grid_latent) {
@@ -1874,6 +1906,9 @@ int sgh_plan_destroy(sgh_plan* p) {
   if (p->graph) cudaGraphDestroy(p->graph);
   if (p->cs1) cudaStreamDestroy(p->cs1);
   if (p->cs2) cudaStreamDestroy(p->cs2);
+  if (p->fs) cudaStreamDestroy(p->fs);
+  for (cudaEvent_t e : p->fe)
+    if (e) cudaEventDestroy(e);
   if (p->host_out) cudaFreeHost(p->host_out);
   delete p;
   return SGH_OK;
@@ -1948,6 +1983,10 @@ int sgh_plan_bind(sgh_plan* p, void* workspace, uint64_t bytes, void* stream) {
   SGH_CK(cudaStreamSynchronize(s));
   SGH_CK(cudaStreamCreateWithFlags(&p->cs1, cudaStreamNonBlocking));
   SGH_CK(cudaStreamCreateWithFlags(&p->cs2, cudaStreamNonBlocking));
+  if (h.box) {
+    SGH_CK(cudaStreamCreateWithFlags(&p->fs, cudaStreamNonBlocking));
+    for (cudaEvent_t& e : p->fe) SGH_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  }
   const int rc = capture(p);
   if (rc) return rc;
   p->bound = true;
