@@ -998,6 +998,22 @@ bool program_affine(const sgh_program& p, double* A, double* B) {
   return std::isfinite(*A) && std::isfinite(*B);
 }
 
+// Whether a program is a + b T + c T^2 written as a +- b * T +- c * T**2, with
+// its coefficients (signs folded into b and c, which changes no bit).
+bool program_quadratic(const sgh_program& p, double* A, double* B, double* C2) {
+  if (p.n_ops != 15) return false;
+  const int32_t* o = p.ops;
+  const auto sign = [](int op) { return op == SGH_OP_ADD || op == SGH_OP_SUB; };
+  if (o[0] != SGH_OP_CONST || o[2] != SGH_OP_CONST || o[4] != SGH_OP_T || o[5] != SGH_OP_MUL || !sign(o[6]) ||
+      o[7] != SGH_OP_CONST || o[9] != SGH_OP_T || o[10] != SGH_OP_CONST || o[12] != SGH_OP_POW ||
+      o[13] != SGH_OP_MUL || !sign(o[14]) || p.consts[o[11]] != 2.0)
+    return false;
+  *A = p.consts[o[1]];
+  *B = o[6] == SGH_OP_ADD ? p.consts[o[3]] : -p.consts[o[3]];
+  *C2 = o[14] == SGH_OP_ADD ? p.consts[o[8]] : -p.consts[o[8]];
+  return true;
+}
+
 // ---- enqueue helpers (used both for graph capture and for direct calls) ----
 
 template <class Epi>
@@ -1758,6 +1774,7 @@ int sgh_plan_create(const sgh_config* cfg, sgh_plan** out) {
   h.area_factor = c.area_factor;
   h.omega = c.omega;
   h.tol = c.tol;
+  h.two = 2.0;
   if (box) {
     // FineMeshState.__init__ (physics/spectral_state.py:189-227), in its operation order
     const double r = (double)c.box_refinement;
@@ -1787,7 +1804,8 @@ int sgh_plan_create(const sgh_config* cfg, sgh_plan** out) {
     h.prog[P_C_SOLID] = c.c_solid;
     h.prog[P_C_LIQUID] = c.c_liquid;
     for (int i = 0; i < P_COUNT; ++i)
-      h.affine[i] = program_affine(h.prog[i], &h.aff_a[i], &h.aff_b[i]) ? 1 : 0;
+      h.affine[i] = program_affine(h.prog[i], &h.aff_a[i], &h.aff_b[i]) ? 1
+                    : program_quadratic(h.prog[i], &h.aff_a[i], &h.aff_b[i], &h.aff_c[i]) ? 2 : 0;
   }
 
   p->nparts_relax = std::min(RELAX_BLOCKS_MAX, cdiv(h.V, EW_THREADS));
