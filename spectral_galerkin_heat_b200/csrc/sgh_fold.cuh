@@ -321,6 +321,17 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// One element, global -> shared, asynchronously (4 or 8 bytes).
+template <class W>
+__device__ __forceinline__ void copy_async(W* dst, const W* src) {
+  if (sizeof(W) == 8) {
+    cp_async8(dst, src, 8);
+  } else {
+    const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(src));
+  }
+}
+
 // All threads of all CTAs of the cluster. The result is complete on rank 0,
 // thread 0. bad: this CTA's operands are invalid (an expired wait): its
 // partials become NaN and the step ends non-finite. KEEPM: the packed matrices
@@ -356,18 +367,21 @@ __device__ FaceResult face_step(const FaceShape& f, const FaceJob<W>& J, double*
   const double* pyf = KEEPM ? sm + f.o_m + 2 * nxp : J.pyf;
   const double* pyi = KEEPM ? sm + f.o_m + 2 * nxp + nyp : J.pyi;
 
-  if (keepw) {  // this CTA's columns of the face sums and weights, in position order
+  if (keepw) {
+    // this CTA's columns of the face sums and weights, in position order, copied
+    // while the laser flux and the first passes run
     for (int p = warp; p < ny; p += NW) {
       const size_t g0 = (size_t)mode_at(p, ny) * nx;
       for (int c = lane; c < nc; c += 32) {
         const size_t gi = g0 + mode_at(c0 + c, nx);
         const int li = p * ldc + c;
-        sw[li] = J.Zt[gi];
-        sw[wstride + li] = J.Wtt[gi];
-        sw[2 * wstride + li] = J.Yt[gi];
-        sw[3 * wstride + li] = J.Qtt[gi];
+        copy_async(&sw[li], J.Zt + gi);
+        copy_async(&sw[wstride + li], J.Wtt + gi);
+        copy_async(&sw[2 * wstride + li], J.Yt + gi);
+        copy_async(&sw[3 * wstride + li], J.Qtt + gi);
       }
     }
+    cp_async_commit();
   }
   // laser flux, warm-start shift (solvers/spectral.py:273-306); sums of q_las per 32 cells of a row
   const int XC = (nx + 31) / 32;
@@ -446,6 +460,7 @@ __device__ FaceResult face_step(const FaceShape& f, const FaceJob<W>& J, double*
     pass(std::integral_constant<int, 0>{}, pxf, nx, xt, 1, ldr, nr, to_columns);
     sync_all();
     pass(std::integral_constant<int, 0>{}, pyf, ny, xc, ldc, 1, nc, keep_col);
+    if (res.iter < 0) cp_async_wait<0>();  // the weights of this thread's copies have landed
     __syncthreads();
     // 8 positions x 8 columns per warp, two elements per lane
     for (int task = warp; task < PT * vt_n; task += NW) {
