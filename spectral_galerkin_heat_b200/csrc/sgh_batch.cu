@@ -290,9 +290,20 @@ kb_slot_start(BView v, int s, R* a, const R* K, const R* KK, double* q_evold, do
   const BSlot& sl = v.slot[s];
   const long long i = (long long)blockIdx.x * BT + threadIdx.x;
   const R a0 = (R)(sl.T0 * sqrt(sl.Lx * sl.Ly * sl.Lz));
-#pragma unroll
-  for (int c = 0; c < 4; ++c)
-    if (4 * i + c < sl.V) a[sl.vol + 4 * i + c] = 4 * i + c == 0 ? a0 : (R)0;
+  {  // sl.vol is a multiple of 4 elements: 16-byte stores
+    R* o = a + sl.vol + 4 * i;
+    const R first = i == 0 ? a0 : (R)0;
+    if (4 * i + 3 < sl.V) {
+      if constexpr (TAB) {
+        *reinterpret_cast<float4*>(o) = make_float4(first, 0.0f, 0.0f, 0.0f);
+      } else {
+        reinterpret_cast<double2*>(o)[0] = make_double2(first, 0.0);
+        reinterpret_cast<double2*>(o)[1] = make_double2(0.0, 0.0);
+      }
+    } else {
+      for (int c = 0; c < 4 && 4 * i + c < sl.V; ++c) o[c] = c == 0 ? first : (R)0;
+    }
+  }
   if (i < sl.S) {
     q_evold[sl.face + i] = 0.0;
     sigma[sl.face + i] = 0.0;
