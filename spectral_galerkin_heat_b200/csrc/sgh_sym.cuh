@@ -20,10 +20,13 @@
 // CTAs per SM cover each other's prologue and epilogue. Results leave through
 // shared memory along the output's contiguous direction, whose strides the
 // caller gives, so that an array can be written transposed.
-// Measured on a B200: the 512 x 256 x 64 node field 443 us (16 TFLOP/s of halved
-// work) against 667 with full contractions and a transposing copy; DCT-II and
+// Measured on a B200: the 512 x 256 x 64 node field 390 us (18 TFLOP/s of halved
+// work; 443 with the middle output as one more pair) against 667 with full
+// contractions and a transposing copy; DCT-II and
 // DCT-III of a 96 x 60 x 100 volume 66 us against 86.
 #pragma once
+#include <algorithm>
+
 #include "sgh_axis.cuh"
 
 namespace sgh {
@@ -45,7 +48,7 @@ struct Lay {
   static constexpr int XSIZE = CONTIG ? (FWD ? 2 * BC * LDX : BC * LDX) : 2 * KP * LDX;
   static constexpr int STAGE = MR * LDM + XSIZE;
   static constexpr int TILE = 2 * BJ * (BC + 1);  // epilogue
-  static constexpr int BYTES = (SYM_STAGES * STAGE > TILE ? SYM_STAGES * STAGE : TILE) * 8;
+  static constexpr int BYTES = (SYM_STAGES * STAGE > TILE + THREADS ? SYM_STAGES * STAGE : TILE + THREADS) * 8;
 };
 
 struct Args {
@@ -64,7 +67,14 @@ __global__ void __launch_bounds__(THREADS, 2) k_sym(Args q) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3, wm = warp >> 2, wn = warp & 3;
   const int N = q.N, Nout = q.Nout, B = q.B, ncol = q.A * B;
-  const int H = (Nout + 1) / 2, h = (N + 1) / 2;  // output pairs; forward: slices kept
+  // output pairs (the middle output of an odd inverse form is not one), slices a
+  // forward pass keeps
+  const int H = FWD ? (Nout + 1) / 2 : Nout / 2, h = (N + 1) / 2;
+  // The middle output contracts the even slices only. It is summed by the CUDA
+  // cores of the last row of CTAs from the staged slices: as one more pair it would
+  // cost a tile of 32 (N / 2 + 1 pairs of a node matrix: 3 tiles of 32 for 64).
+  const bool mid = !FWD && (Nout & 1) && blockIdx.y == gridDim.y - 1;
+  double msum = 0.0;
   const int c0 = blockIdx.x * BC, j0 = blockIdx.y * BJ;
   const int nch = (h + KP - 1) / KP;
   const bool vm = (N % 2 == 0) && (reinterpret_cast<uintptr_t>(q.Mat) % 16 == 0) && !(FWD && (h & 1));
@@ -183,6 +193,14 @@ __global__ void __launch_bounds__(THREADS, 2) k_sym(Args q) {
     else cp_async_commit();
     const double* Ms = sy + (ch % SYM_STAGES) * L::STAGE;
     const double* Xs = Ms + L::MR * L::LDM;
+    if (mid) {
+      const int col = tid % BC;
+#pragma unroll
+      for (int i = 0; i < KP * BC / THREADS; ++i) {
+        const int s = 2 * (tid / BC + (THREADS / BC) * i), n = 2 * KP * ch + s;
+        if (n < N) msum = fma(__ldg(q.Mat + (size_t)(Nout / 2) * N + n), CONTIG ? Xs[col * L::LDX + s] : Xs[s * L::LDX + col], msum);
+      }
+    }
 #pragma unroll
     for (int k8 = 0; k8 < KP; k8 += 8) {
       double fe[4], fo[4];
@@ -240,7 +258,15 @@ __global__ void __launch_bounds__(THREADS, 2) k_sym(Args q) {
       tile[(FWD ? 2 * jr : jr) * LDT + col] = FWD ? ae[v][i] : ae[v][i] + ao[v][i];
       tile[(FWD ? 2 * jr + 1 : 2 * BJ - 1 - jr) * LDT + col] = FWD ? ao[v][i] : ae[v][i] - ao[v][i];
     }
+  if (mid) tile[L::TILE + tid] = msum;
   __syncthreads();
+  if (mid && tid < BC && c0 + tid < ncol) {
+    double s = 0.0;
+#pragma unroll
+    for (int i = 0; i < THREADS / BC; ++i) s += tile[L::TILE + BC * i + tid];
+    const int c = c0 + tid, a = CONTIG ? c : c / B, b = CONTIG ? 0 : c - a * B;
+    q.out[a * q.sa + (Nout / 2) * q.sk + b] = s;
+  }
   for (int e = tid; e < 2 * BJ * BC; e += THREADS) {
     const int r = q.kfast ? e % (2 * BJ) : e / BC, cr = q.kfast ? e / (2 * BJ) : e % BC;
     const int c = c0 + cr;
@@ -255,7 +281,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_sym(Args q) {
     } else {
       const int j = j0 + 2 * BJ - 1 - r;
       k = Nout - 1 - j;
-      ok = ok && j < H && k != j;
+      ok = ok && j < H;
     }
     if (ok) {
       const int a = CONTIG ? c : c / B, b = CONTIG ? 0 : c - a * B;
@@ -274,7 +300,7 @@ inline void launch_one(const Args& q, cudaStream_t st) {
     return true;
   }();
   (void)attr;
-  const int H = (q.Nout + 1) / 2;
+  const int H = FWD ? (q.Nout + 1) / 2 : std::max(1, q.Nout / 2);
   const dim3 grid((unsigned)(((long long)q.A * q.B + BC - 1) / BC), (unsigned)((H + BJ - 1) / BJ));
   launch_pdl(k_sym<CONTIG, FWD>, grid, THREADS, L::BYTES, st, q);
 }
