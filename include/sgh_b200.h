@@ -82,7 +82,10 @@ typedef struct {
   /* SGH_PRECISION_FP64, or SGH_PRECISION_MIXED: every DCT contraction of the
    * step as split-BF16 products on the tensor cores (hi/lo operands, three
    * products, FP32 accumulation) and the modal iterates rounded to FP32 at
-   * every write; the latent source across the solidus-liquidus band, the
+   * every write -- except where the volume form runs fused (grid mode, one
+   * property branch for both phases, slabs that fit a thread-block cluster):
+   * there the loop's contractions and iterates are FP64, which is faster and more
+   * exact, and the committed modes are rounded to FP32; the latent source across the solidus-liquidus band, the
    * property correction, the face fluxes, the Picard norms and the
    * coefficient tables stay FP64. SGH_PRECISION_FP32: the same with FP32
    * contractions on the CUDA cores instead. */
@@ -114,7 +117,8 @@ typedef struct {
    * Chosen per (nx, ny, nz) by the autotuner (autotune.py). Batches ignore it. */
   int32_t axis_min_ctas;
   /* 0: passes large enough run on the FP64 tensor cores (mma.sync .f64);
-   * 1: every pass runs on the CUDA-core FP64 kernels (for comparison). */
+   * 1: every pass runs on the CUDA-core FP64 kernels (for comparison), and the
+   * volume form is not fused. A face-space step in a cluster has no passes. */
   int32_t axis_cuda_cores;
   /* Laser-following refined sub-box (FineMeshParams, core/parameters.py:391-410;
    * FineMeshState, physics/spectral_state.py:166-239). box = 1 selects box
@@ -327,7 +331,8 @@ int sgh_dctn(int32_t kind, int32_t ndim, const int32_t* shape, const double* in,
  * instance per solver (solvers/spectral.py:219-543).
  * ------------------------------------------------------------------------ */
 #define SGH_PRECISION_MIXED 1   /* FP32 modes and K/KK (computed in FP64); face contractions in
-                                   split-BF16 on the tensor cores; FP64 faces and norms */
+                                   split-BF16 on the tensor cores (slots with a Picard loop and
+                                   a face of up to 32768 cells: FP64); FP64 faces and norms */
 
 typedef struct sgh_batch sgh_batch;
 

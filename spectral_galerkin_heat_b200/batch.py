@@ -8,6 +8,10 @@ stage. Each slot runs the reference step (``solvers/spectral.py:219-543``) in
 its face-space form, so the supported physics is laser + evaporation without
 convection, latent heat or a T-dependent model.
 
+Slots in FP64, and mixed slots with a Picard loop, whose face fits a
+thread-block cluster run their whole face step in one kernel with FP64
+contractions; the choice depends on the slot alone.
+
 ``precision="fp64"`` keeps the modes and K/KK in FP64; ``precision="mixed"``
 stores the modes in FP32 (K and KK formed from FP64 1-D tables), with FP64 face
 fields (fluxes, sigma, surface) and norms and FP32 face sums and weights,

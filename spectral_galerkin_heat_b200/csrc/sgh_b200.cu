@@ -19,6 +19,12 @@
 // synchronisation per Picard iteration, where the reference issues ~20 array
 // operations and one device->host float() per iteration
 // (solvers/spectral.py:386-499).
+//
+// Two forms replace the loop's pass-per-axis kernels where they fit: face-space
+// plans without convection run the whole step -- Picard loop included -- in one
+// cluster kernel between two volume passes (sgh_fold.cuh, k_face_run), and
+// grid-mode volume plans run an iteration in five fused kernels
+// (sgh_volume.cuh). cluster and slab of sgh_plan say which form a plan takes.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -16,6 +16,11 @@
 // still iterating; converged (or inactive) slots skip every kernel of the
 // body, so a slot's result does not depend on what else is in the batch.
 //
+// Slots whose face fits a thread-block cluster (slot_cluster: FP64 slots, and
+// mixed slots with a Picard loop) run laser flux, Picard loop, convergence test and
+// surface commit in one kernel each step instead (kb_face_cluster, sgh_fold.cuh),
+// in FP64 in either precision; the stages above then launch for the others only.
+//
 // Volume state is FP64 modes with stored K and KK (plain), or FP32 modes only
 // (mixed: K and KK formed in registers from per-axis FP64 tables, the mode
 // update in FP32). Face fields and norms are FP64 in both; the face sums and

@@ -234,9 +234,11 @@ class B200SpectralSolver(HeatSolver):
     """Spectral-Galerkin heat step on one B200 (grid or box mode).
 
     ``precision="fp64"`` (default) is the plain form, FP64 throughout.
-    ``precision="mixed"`` runs every DCT contraction of the step as split-BF16
-    products on the tensor cores (tcgen05, FP32 accumulation) and keeps the
-    modal iterates rounded to FP32; the latent source across the
+    ``precision="mixed"`` keeps FP32 modes. Grid-mode volume steps whose slabs
+    fit a thread-block cluster (and whose properties have one branch for both
+    phases) run in FP64 and round the committed modes; every other step runs its
+    DCT contractions as split-BF16 products on the tensor cores (tcgen05, FP32
+    accumulation) and rounds the modal iterates to FP32 at every write; the latent source across the
     solidus-liquidus band, the property correction, the face fluxes, the
     Picard norms and the coefficient tables stay FP64. ``precision="fp32"``
     is the same with FP32 contractions on the CUDA cores (the FP32 arm of the
