@@ -1922,8 +1922,7 @@ int capture(sgh_batch* B) {
 }
 
 // CTAs of the cluster that runs a slot's face step, 0 for the multi-kernel path.
-// A rule on the slot's own shape and Picard cap, so that its results do not
-// depend on the rest of the batch. FP64: wherever the face fits (18 serving
+// A rule on the slot's shape and Picard cap and on the load. FP64: wherever the face fits (18 serving
 // slots up to 256 x 128: 1.71 -> 0.86 ms for 6 steps). Mixed: Picard loops up to
 // 32768 elements, where the launches and epilogue latencies of the tensor-core
 // kernels dominate (32 uneven slots, 3 steps of 30 iterations: 7.6 -> 2.4 ms; 4
@@ -1931,10 +1930,39 @@ int capture(sgh_batch* B) {
 // tensor-core kernels take all slots of a batch at once and are faster (48
 // serving slots: 1.45 ms against 1.50 with the 64 x 32 faces on clusters, 1.85
 // with every face up to 256 x 128).
-int slot_cluster(const sgh_config& c, int precision) {
-  if (precision != SGH_PRECISION_MIXED) return fold::cluster_size<double>(c.nx, c.ny);
-  if (c.max_iter <= 1 || (long)c.nx * c.ny > 32768) return 0;
-  return fold::cluster_size<float>(c.nx, c.ny);
+//
+// The load, in waves of FACE_SHARE elements on every SM, decides as well. Picard
+// batches of 128 x 64 to 256 x 128 faces (13,200 elements on average, mixed), time
+// of three steps:
+//   slots                        16    32    64    96   128   256   512
+//   waves                       0.7   1.4   2.8   4.2   5.6    11    22
+//   2048 elements a CTA  ms    1.57  2.31  3.98  5.73  7.49  13.8  27.3
+//   4096 elements a CTA  ms    2.62  3.16  4.09  5.31  6.60  11.1  21.6
+//   tensor-core kernels  ms    6.57  7.71  7.78  8.38  8.94  11.2  17.2
+// FP64 crosses from 2048 to 4096 at the same place (64 slots 4.33 against 4.44,
+// 128: 8.33 against 7.45) and has no third form. The share of a CTA does not
+// change a bit of the result; the tensor-core kernels differ from the clusters
+// within the mixed form's bound.
+// Faces below CROWD_WIDE_FACE elements stay on clusters: most of a tensor-core
+// tile would be padding (2048 ragged slots of 24-64 columns, 8 steps: 28 against
+// 69 ms); with 64 x 32 faces left there too 256 slots take 11.5 ms, not 10.7.
+constexpr double CROWD = 3.0, CROWD_WIDE = 10.0;
+constexpr long CROWD_WIDE_FACE = 2048;
+int slot_cluster(const sgh_config& c, int precision, double waves) {
+  const bool mixed = precision == SGH_PRECISION_MIXED;
+  const long S = (long)c.nx * c.ny;
+  if (mixed && (c.max_iter <= 1 || S > 32768 || (waves > CROWD_WIDE && S >= CROWD_WIDE_FACE))) return 0;
+  if (waves > CROWD)
+    return mixed ? fold::cluster_size_crowded<float>(c.nx, c.ny) : fold::cluster_size_crowded<double>(c.nx, c.ny);
+  return mixed ? fold::cluster_size<float>(c.nx, c.ny) : fold::cluster_size<double>(c.nx, c.ny);
+}
+
+// Times the cluster slots of a batch fill the chip, at FACE_SHARE elements a CTA.
+double slot_waves(const sgh_config* cfgs, int n, int precision) {
+  double e = 0;
+  for (int i = 0; i < n; ++i)
+    if (slot_cluster(cfgs[i], precision, 0)) e += (double)cfgs[i].nx * cfgs[i].ny;
+  return e / (148.0 * fold::FACE_SHARE);
 }
 
 struct LayoutB {
@@ -1996,12 +2024,13 @@ int sgh_batch_create(const sgh_config* cfgs, int32_t n, int32_t precision, sgh_b
     moff += 2LL * kv.first * kv.first;
   }
   B->mat_elems = moff;
+  const double waves = slot_waves(cfgs, n, precision);
   std::map<int, long long> mplane;
   if (precision == SGH_PRECISION_MIXED) {
     long long po = 0;
     std::map<int, int> wide;  // lengths of the slots on the tensor-core path
     for (int i = 0; i < n; ++i)
-      if (!slot_cluster(cfgs[i], precision)) wide[cfgs[i].nx] = wide[cfgs[i].ny] = 1;
+      if (!slot_cluster(cfgs[i], precision, waves)) wide[cfgs[i].nx] = wide[cfgs[i].ny] = 1;
     for (auto& kv : wide) {
       // per N: forward, inverse in 128-row chunks (the A operand of the
       // y-pass and the B operand of the x-pass alike)
@@ -2035,7 +2064,7 @@ int sgh_batch_create(const sgh_config* cfgs, int32_t n, int32_t precision, sgh_b
     sl.mx = (int)mats[c.nx];
     sl.my = (int)mats[c.ny];
     sl.nblk = cdivl(sl.S, BT);
-    sl.cl = slot_cluster(c, precision);
+    sl.cl = slot_cluster(c, precision, waves);
     if (sl.cl)
       for (int q = 0; q < 4; ++q) sl.fold[q] = fold_at(q < 2 ? c.nx : c.ny) + (q & 1) * (long long)fold::pack_doubles(q < 2 ? c.nx : c.ny);
     sl.rblk0 = B->tot_rblk;

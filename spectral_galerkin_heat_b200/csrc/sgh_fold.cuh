@@ -289,6 +289,16 @@ __host__ inline int cluster_size(int nx, int ny) {
     if (face_shape<W>(nx, ny, n).bytes <= FACE_SMEM_MAX - 512) return n;
   return 0;
 }
+// Cluster size of a face among so many that the chip is filled several times
+// over: the fewest CTAs of at most FACE_SHARE_CROWDED elements each that hold it,
+// since waves of clusters then count and the passes' latency does not.
+constexpr long FACE_SHARE = 2048, FACE_SHARE_CROWDED = 4096;
+template <class W>
+__host__ inline int cluster_size_crowded(int nx, int ny) {
+  for (int n = 1; n <= FACE_MAX_CLUSTER; n *= 2)
+    if ((long)nx * ny <= FACE_SHARE_CROWDED * n && face_shape<W>(nx, ny, n).bytes <= FACE_SMEM_MAX - 512) return n;
+  return cluster_size<W>(nx, ny);
+}
 // Threads of a face kernel: eight warps cover the tasks of a small share
 // (64 x 32 on 4 CTAs: 407 us with 256 or 512 threads, 437 with 128), larger
 // ones want sixteen (256 x 128: 884 us with 256, 749 with 512, at 8 CTAs).

@@ -92,3 +92,31 @@ def test_steps_one_by_one_equal_a_run_and_wide_slots_share_a_batch():
         assert np.array_equal(alone.modes(0).cpu().numpy(), mix.modes(i).cpu().numpy())
         alone.close()
     mix.close()
+
+
+@pytest.mark.parametrize("count,precision", [(30, "fp64"), (600, "fp64"), (600, "mixed"), (2000, "mixed")])
+def test_crowded_batches(count, precision):
+    """Face shares of a lightly and a heavily loaded batch: a slot among many
+    (shares of up to 4096 elements; above 10 waves the tensor-core kernels from 2048 on)
+    against the same slot alone. FP64 and mixed clusters to the bit; the
+    tensor-core kernels to 2e-4, the bound of the mixed form on each side."""
+    from spectral_galerkin_heat_b200.batch import BatchSolver
+    steps = 2
+    shapes = [(64, 33), (47, 32), (100, 60)]
+    ctxs = [_ctx(nx, ny, 5, steps, cap=8) for nx, ny in shapes]
+    waves = count / 3 * sum(x * y for x, y in shapes) / (148 * 2048)
+    b = BatchSolver([ctxs[i % 3] for i in range(count)], precision)
+    for i in range(count):
+        b.start(i, steps)
+    b.step(steps)
+    for i in (0, count // 2 // 3 * 3 + 1, count - 1 - count % 3):
+        one = BatchSolver([ctxs[i % 3]], precision)
+        one.start(0, steps)
+        one.step(steps)
+        x, y = b.modes(i).cpu().numpy(), one.modes(0).cpu().numpy()
+        if precision == "mixed" and waves > 10 and i % 3 != 1:
+            assert rel_l2(x, y) < 2e-4
+        else:
+            assert np.array_equal(x, y)
+        one.close()
+    b.close()
