@@ -38,6 +38,7 @@
 #include "sgh_b200.h"
 #include "sgh_device.cuh"
 #include "sgh_fold.cuh"
+#include "sgh_limits.h"
 #include "sgh_sym.cuh"
 #include "sgh_volume.cuh"
 
@@ -1359,7 +1360,7 @@ void enqueue_column(sgh_plan* p, const double* in, double* out, cudaStream_t s) 
   q.T = p->d(p->o_vol); q.kp = p->d(p->o_kp);
   q.Tprev_out = p->d(p->o_Tprev); q.T_surf = p->d(p->o_Tsurf); q.q_evap_old = p->d(p->o_qevold);
   q.partials = p->d(p->o_psurf);
-  (void)cudaFuncSetAttribute(vol::k_column<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, f.bytes);
+  SGH_CK_VOID(kernel_limits(reinterpret_cast<const void*>(vol::k_column<MODE>), f.bytes));
   launch_pdl(vol::k_column<MODE>, dim3(cdiv(h.S, f.cc)), vol::COL_THREADS, f.bytes, s, f, q);
   ++g_launches;
 }
@@ -2094,6 +2095,7 @@ int sgh_step(sgh_plan* p, const sgh_laser* laser, sgh_step_out* out, void* strea
   if (p->cluster) {  // three launches: cheaper than a graph with a conditional node
     enqueue_fs_volume<false, true>(p, s, *laser, nullptr, nullptr, 1);
     enqueue_face_run(p, s, 0, 0);
+    SGH_CK(cudaGetLastError());  // no commit with the sigma of another step
     enqueue_fs_volume<true, false>(p, s, sgh_laser{}, nullptr, nullptr, 0);
     SGH_CK(cudaGetLastError());
     SGH_CK(cudaStreamSynchronize(s));

@@ -31,6 +31,7 @@
 
 #include "sgh_axis.cuh"
 #include "sgh_device.cuh"
+#include "sgh_limits.h"
 #include "sgh_umma.cuh"
 
 namespace sgh {
@@ -634,12 +635,8 @@ template <class... KArgs, class... Args>
 inline cudaError_t launch_cluster(void (*kernel)(KArgs...), int ctas, int n, int threads, int smem, bool pdl,
                                   cudaStream_t st,
                                   Args&&... args) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const cudaError_t e = kernel_limits(reinterpret_cast<const void*>(kernel), smem, n > 8);
   if (e != cudaSuccess) return e;
-  if (n > 8) {
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(threads);
