@@ -1360,7 +1360,7 @@ void enqueue_column(sgh_plan* p, const double* in, double* out, cudaStream_t s) 
   q.T = p->d(p->o_vol); q.kp = p->d(p->o_kp);
   q.Tprev_out = p->d(p->o_Tprev); q.T_surf = p->d(p->o_Tsurf); q.q_evap_old = p->d(p->o_qevold);
   q.partials = p->d(p->o_psurf);
-  SGH_CK_VOID(kernel_limits(reinterpret_cast<const void*>(vol::k_column<MODE>), f.bytes));
+  SGH_CK_VOID(kernel_limits(reinterpret_cast<const void*>(vol::k_column<MODE>), vol::COL_SMEM_MAX));
   launch_pdl(vol::k_column<MODE>, dim3(cdiv(h.S, f.cc)), vol::COL_THREADS, f.bytes, s, f, q);
   ++g_launches;
 }
@@ -1578,7 +1578,7 @@ int fused_slab(const sgh_plan* p) {
   if (h.box || p->face_space || !(h.grid_latent || h.prop_corr)) return 0;
   if (p->cfg.precision == SGH_PRECISION_FP32 || p->cfg.axis_cuda_cores) return 0;
   if (h.prop_corr && phase_branches(p->cfg)) return 0;
-  if (vol::col_shape(h.nx, h.ny, h.nz).bytes > 200 * 1024) return 0;
+  if (vol::col_shape(h.nx, h.ny, h.nz).bytes > vol::COL_SMEM_MAX) return 0;
   return vol::slab_cluster(h.nx, h.ny, h.nz);
 }
 

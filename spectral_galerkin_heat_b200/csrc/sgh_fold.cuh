@@ -231,7 +231,7 @@ __device__ __forceinline__ void fold_pass(const double* P, int N, const double* 
 // the cluster size or on the other instances of a launch.
 constexpr int FACE_THREADS = 512;  // most threads of a face kernel
 constexpr int FACE_MAX_CLUSTER = 16;
-constexpr int FACE_SMEM_MAX = 227 * 1024;
+constexpr int FACE_SMEM_MAX = 227 * 1024;  // shapes leave 512 bytes of it to the kernels' static arrays
 
 // Row stride of a shared array: at least n, 4 or 12 mod 16 doubles (fragment
 // reads along and across rows then hit all banks).
@@ -635,7 +635,7 @@ template <class... KArgs, class... Args>
 inline cudaError_t launch_cluster(void (*kernel)(KArgs...), int ctas, int n, int threads, int smem, bool pdl,
                                   cudaStream_t st,
                                   Args&&... args) {
-  const cudaError_t e = kernel_limits(reinterpret_cast<const void*>(kernel), smem, n > 8);
+  const cudaError_t e = kernel_limits(reinterpret_cast<const void*>(kernel), FACE_SMEM_MAX - 512, true);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctas);

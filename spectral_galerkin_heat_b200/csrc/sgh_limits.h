@@ -4,9 +4,10 @@
 // belong to a kernel (per device), not to a launch: any host thread that lowers a limit
 // can make another thread's launch of the same kernel fail, and a limit raised
 // on one device says nothing about the next. kernel_limits() therefore only ever
-// raises them, once per kernel, device and size, under a lock; every launch with
-// more than 48 KB of dynamic shared memory whose size depends on the problem
-// calls it first. About 30 ns when there is nothing to raise.
+// raises them, once per kernel, device and size, under a lock, and every launch
+// calls it first. Callers pass the largest size that the kernel is ever launched
+// with, so that the one call to the runtime precedes every launch of the kernel on
+// that device and none runs beside it. About 30 ns when there is nothing to raise.
 #pragma once
 #include <cuda_runtime_api.h>
 

@@ -419,6 +419,8 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) k_slab(SlabShape f, SlabArgs 
   }
 }
 
+constexpr int COL_SMEM_MAX = 200 * 1024;  // largest dynamic shared memory of a column kernel
+
 struct ColShape {
   int nx, ny, nz, cc, ld, bytes;
 };
