@@ -10,9 +10,8 @@ convection, latent heat or a T-dependent model.
 
 Slots in FP64, and mixed slots with a Picard loop, whose face fits a
 thread-block cluster run their whole face step in one kernel with FP64
-contractions; the choice depends on the slot, and in batches of several
-hundred mixed Picard slots on the load: there the larger faces take the tensor-core
-kernels, within the same bound.
+contractions. The choice depends on the slot alone (its face and its Picard
+cap), so a slot gives the same bits in every batch.
 
 ``precision="fp64"`` keeps the modes and K/KK in FP64; ``precision="mixed"``
 stores the modes in FP32 (K and KK formed from FP64 1-D tables), with FP64 face

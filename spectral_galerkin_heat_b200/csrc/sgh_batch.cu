@@ -1922,7 +1922,10 @@ int capture(sgh_batch* B) {
 }
 
 // CTAs of the cluster that runs a slot's face step, 0 for the multi-kernel path.
-// A rule on the slot's shape and Picard cap and on the load. FP64: wherever the face fits (18 serving
+// Whether a slot takes a cluster depends on its own shape and Picard cap only:
+// the two paths round differently, and a slot's result is the same alone, in
+// any batch, over any number of lanes and after it moved to another batch.
+// FP64: wherever the face fits (18 serving
 // slots up to 256 x 128: 1.71 -> 0.86 ms for 6 steps). Mixed: Picard loops up to
 // 32768 elements, where the launches and epilogue latencies of the tensor-core
 // kernels dominate (32 uneven slots, 3 steps of 30 iterations: 7.6 -> 2.4 ms; 4
@@ -1931,7 +1934,8 @@ int capture(sgh_batch* B) {
 // serving slots: 1.45 ms against 1.50 with the 64 x 32 faces on clusters, 1.85
 // with every face up to 256 x 128).
 //
-// The load, in waves of FACE_SHARE elements on every SM, decides as well. Picard
+// The load, in waves of FACE_SHARE elements on every SM, decides only the size of
+// the cluster, which does not change a bit of the result. Picard
 // batches of 128 x 64 to 256 x 128 faces (13,200 elements on average, mixed), time
 // of three steps:
 //   slots                        16    32    64    96   128   256   512
@@ -1940,18 +1944,12 @@ int capture(sgh_batch* B) {
 //   4096 elements a CTA  ms    2.62  3.16  4.09  5.31  6.60  11.1  21.6
 //   tensor-core kernels  ms    6.57  7.71  7.78  8.38  8.94  11.2  17.2
 // FP64 crosses from 2048 to 4096 at the same place (64 slots 4.33 against 4.44,
-// 128: 8.33 against 7.45) and has no third form. The share of a CTA does not
-// change a bit of the result; the tensor-core kernels differ from the clusters
-// within the mixed form's bound.
-// Faces below CROWD_WIDE_FACE elements stay on clusters: most of a tensor-core
-// tile would be padding (2048 ragged slots of 24-64 columns, 8 steps: 28 against
-// 69 ms); with 64 x 32 faces left there too 256 slots take 11.5 ms, not 10.7.
-constexpr double CROWD = 3.0, CROWD_WIDE = 10.0;
-constexpr long CROWD_WIDE_FACE = 2048;
+// 128: 8.33 against 7.45). Past some 10 waves the tensor-core kernels would be the
+// faster ones for mixed slots; they are not taken there, for the reason above.
+constexpr double CROWD = 3.0;
 int slot_cluster(const sgh_config& c, int precision, double waves) {
   const bool mixed = precision == SGH_PRECISION_MIXED;
-  const long S = (long)c.nx * c.ny;
-  if (mixed && (c.max_iter <= 1 || S > 32768 || (waves > CROWD_WIDE && S >= CROWD_WIDE_FACE))) return 0;
+  if (mixed && (c.max_iter <= 1 || (long)c.nx * c.ny > 32768)) return 0;
   if (waves > CROWD)
     return mixed ? fold::cluster_size_crowded<float>(c.nx, c.ny) : fold::cluster_size_crowded<double>(c.nx, c.ny);
   return mixed ? fold::cluster_size<float>(c.nx, c.ny) : fold::cluster_size<double>(c.nx, c.ny);

@@ -1,0 +1,54 @@
+"""A slot's result does not depend on the batch around it: mixed and FP64 Picard
+slots alone, among so many that the chip is filled more than ten times over,
+over two lanes, and moved from a small batch into a crowded one in the middle
+of a request give the same bits."""
+import numpy as np
+import pytest
+
+from conftest import make_context
+
+pytestmark = pytest.mark.gpu
+
+STEPS = 3
+COUNT = 100   # 256 x 128 faces on 148 SMs: 10.8 waves of 2048 elements per SM
+
+
+def _ctx(nx, ny):
+    from spectral_galerkin_heat_b200 import workloads
+    from spectral_galerkin_heat_b200.laser import StraightTrack
+    size = (2e-3 * nx / 64, 1e-3 * ny / 32, 0.5e-3)
+    cfg, _ = workloads.straight_track(nx=nx, ny=ny, nz=5, steps=STEPS, size=size)
+    cfg["simulation"].update({"max_picard_iter": 8, "picard_omega": 0.1, "picard_tol": 1e-4})
+    return make_context(cfg, StraightTrack(0.4 * size[0], 0.45 * size[1], 0.8, 0.3, 180.0))
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_slot_alone_in_a_crowd_over_lanes_and_moved(precision):
+    from spectral_galerkin_heat_b200.batch import BatchSolver, LaneBatch
+    ctx = _ctx(256, 128)
+    alone = BatchSolver([ctx], precision)
+    table = alone.laser_table(ctx, 0.0, STEPS)
+    alone.start(0, STEPS, table=table)
+    alone.step(1)
+    state = alone.export_slot(0)
+    alone.step(STEPS - 1)
+    want = alone.modes(0).cpu().numpy()
+    alone.close()
+
+    crowd = BatchSolver([ctx] * COUNT, precision)
+    for i in range(COUNT - 1):
+        crowd.start(i, STEPS, table=table)
+    crowd.step(STEPS)
+    assert np.array_equal(crowd.modes(COUNT // 2).cpu().numpy(), want)
+    crowd.import_slot(COUNT - 1, state, table)
+    crowd.step(STEPS - 1)
+    assert np.array_equal(crowd.modes(COUNT - 1).cpu().numpy(), want)
+    crowd.close()
+
+    lanes = LaneBatch([ctx] * COUNT, precision, lanes=2)
+    for i in range(COUNT):
+        lanes.start(i, STEPS, table=table)
+    lanes.step(STEPS)
+    lanes.synchronize()
+    assert np.array_equal(lanes.modes(COUNT - 1).cpu().numpy(), want)
+    lanes.close()
