@@ -40,8 +40,8 @@ extern "C" {
 #define SGH_STEP_CONVERGED   0   /* Picard residual fell below the tolerance */
 #define SGH_STEP_CAPPED      1   /* hit max_picard_iter                      */
 #define SGH_STEP_NONFINITE   2   /* residual became NaN/Inf; loop stopped    */
-#define SGH_STEP_TC_TIMEOUT  3   /* mixed plan: a bounded tensor-core wait ran
-                                    out; the step's results are not trusted  */
+#define SGH_STEP_TC_TIMEOUT  3   /* a bounded wait of the plan's kernels ran out;
+                                    the step's results are not trusted       */
 
 /* property-expression opcodes (postfix program, see sgh_program) */
 enum {
@@ -296,6 +296,16 @@ int sgh_box_window(sgh_plan* plan, int32_t* i0, void* stream);
  * doubles) and returns after the stream has drained. */
 #define SGH_PICARD_HISTORY_MAX 4096
 int sgh_picard_history(sgh_plan* plan, double* out, int32_t cap, int32_t* n_iter, void* stream);
+
+/* Bound of the data waits of a plan's slab kernels (the fused volume form): at
+ * most `polls` mbarrier polls (0 = the default, 2^22) before the kernel records
+ * the error, waits for its copies in flight (with the default bound) and goes
+ * on; the step's Picard loop then ends and the step reports SGH_STEP_TC_TIMEOUT,
+ * as do later ones until the plan is bound again. stall_test = 1 makes every
+ * such wait run out (needs polls > 0), so that a test can drive the error path
+ * without a fault; 0 for normal stepping. No reference counterpart.
+ * Synchronises the stream. */
+int sgh_plan_set_wait_limit(sgh_plan* plan, uint32_t polls, int32_t stall_test, void* stream);
 
 /* out (nz_box, ny_box, nx_box) = the temperature of modes on the fine box at
  * the current window: reconstruct_temperature_box

@@ -42,7 +42,7 @@ EXPORTED = (
     "sgh_nodal_workspace_bytes", "sgh_nodal_temperature", "sgh_nodal_temperature_xyz", "sgh_points_workspace_bytes",
     "sgh_points_temperature", "sgh_box_geometry", "sgh_box_window", "sgh_box_temperature",
     "sgh_box_project", "sgh_state_flags", "sgh_state_set_flags", "sgh_line_workspace_bytes",
-    "sgh_line_temperature", "sgh_picard_history",
+    "sgh_line_temperature", "sgh_picard_history", "sgh_plan_set_wait_limit",
     "sgh_batch_create", "sgh_batch_destroy", "sgh_batch_workspace_bytes", "sgh_batch_bind",
     "sgh_batch_slot_start", "sgh_batch_slot_stop", "sgh_batch_slot_resume", "sgh_batch_step", "sgh_batch_step_eager",
     "sgh_batch_status",
@@ -184,6 +184,7 @@ def lib() -> C.CDLL:
                                       C.c_double, C.c_double, C.c_double, i32, vp, vp, vp, C.c_uint64, vp],
                                      C.c_int),
             "sgh_state_set_flags": ([vp, i32, vp], C.c_int),
+            "sgh_plan_set_wait_limit": ([vp, C.c_uint32, i32, vp], C.c_int),
             "sgh_picard_history": ([vp, C.POINTER(C.c_double), i32, C.POINTER(i32), vp], C.c_int),
         }
         for name, (args, res) in sig.items():

@@ -29,6 +29,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -2130,6 +2131,20 @@ int sgh_step_eager(sgh_plan* p, const sgh_laser* laser, sgh_step_out* out, void*
   SGH_CK(cudaGetLastError());
   SGH_CK(cudaStreamSynchronize(s));
   if (out) *out = *p->host_out;
+  return SGH_OK;
+}
+
+int sgh_plan_set_wait_limit(sgh_plan* p, uint32_t polls, int32_t stall_test, void* stream) {
+  if (!p) return fail(SGH_ERR_INVALID, "null argument");
+  if (!p->bound) return fail(SGH_ERR_STATE, "plan is not bound");
+  if (stall_test && polls == 0) return fail(SGH_ERR_INVALID, "the wait test needs an explicit poll bound");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const unsigned v[2] = {polls, stall_test ? 1u : 0u};
+  static_assert(offsetof(Ctrl, stall_test) == offsetof(Ctrl, wait_limit) + sizeof(unsigned),
+                "wait_limit and stall_test are adjacent");
+  SGH_CK(cudaMemcpyAsync(reinterpret_cast<char*>(p->ctrl()) + offsetof(Ctrl, wait_limit), v, sizeof(v),
+                         cudaMemcpyHostToDevice, s));
+  SGH_CK(cudaStreamSynchronize(s));
   return SGH_OK;
 }
 

@@ -241,13 +241,29 @@ struct SlabArgs {
   int in_graph;
 };
 
+// Waits for the packed matrices' copies on bar[0], at most lim polls a thread. A
+// thread whose wait ran out (or, with `stall`, that first waited on bar[1], which
+// nothing completes) records it in *err and waits for the copies with the full
+// bound, so that none outlives the CTA.
+__device__ __forceinline__ void slab_operands(uint64_t* bar, unsigned lim, bool stall, int* err) {
+  bool ok = !stall || umma::mbar_wait_bounded(&bar[1], 0u, lim);
+  ok = ok && umma::mbar_wait_bounded(&bar[0], 0u, lim);
+  if (!ok) {
+    atomicExch(err, 1);
+    umma::mbar_wait_bounded(&bar[0], 0u, umma::WAIT_LIMIT);
+  }
+}
+
 // KEEP: the packed matrices are in shared memory (f.keep), else read from L2.
+// An expired wait is recorded in ctrl->umma_err: the step reports
+// SGH_STEP_TC_TIMEOUT, and its relaxations write NaN partials, so that the Picard
+// loop ends there.
 template <int MODE, bool KEEP>
 __global__ void __launch_bounds__(SLAB_THREADS, 1) k_slab(SlabShape f, SlabArgs q) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ __align__(128) double sl_sh[];
-  __shared__ uint64_t bar;
+  __shared__ uint64_t bar[2];
   __shared__ double red[2 * (SLAB_THREADS / 32)];
   constexpr int NW = SLAB_THREADS / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -268,19 +284,22 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) k_slab(SlabShape f, SlabArgs 
   // the previous kernel.
   if (KEEP && tid == 0) {
     double* o = sl_sh + f.o_m;
-    umma::mbar_init(&bar, 1);
+    umma::mbar_init(&bar[0], 1);
+    umma::mbar_init(&bar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    umma::mbar_expect_tx(&bar, 16 * (nxp + nyp));
-    umma::bulk_g2s(o, q.pyf, 8 * nyp, &bar);
-    umma::bulk_g2s(o + nyp, q.pxf, 8 * nxp, &bar);
-    umma::bulk_g2s(o + nyp + nxp, q.pxi, 8 * nxp, &bar);
-    umma::bulk_g2s(o + nyp + 2 * nxp, q.pyi, 8 * nyp, &bar);
+    umma::mbar_expect_tx(&bar[0], 16 * (nxp + nyp));
+    umma::bulk_g2s(o, q.pyf, 8 * nyp, &bar[0]);
+    umma::bulk_g2s(o + nyp, q.pxf, 8 * nxp, &bar[0]);
+    umma::bulk_g2s(o + nyp + nxp, q.pxi, 8 * nxp, &bar[0]);
+    umma::bulk_g2s(o + nyp + 2 * nxp, q.pyi, 8 * nyp, &bar[0]);
   }
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  const unsigned lim = KEEP && q.ctrl->wait_limit ? q.ctrl->wait_limit : umma::WAIT_LIMIT;
+  const bool stall = KEEP && q.ctrl->stall_test != 0;
   if (MODE == SLAB_QM && q.ctrl->iter <= 0) {  // the same for every CTA
     if (KEEP) {
       __syncthreads();
-      umma::mbar_wait_bounded(&bar, 0u);  // no copy outlives the CTA
+      slab_operands(bar, lim, stall, &q.ctrl->umma_err);  // no copy outlives the CTA
     }
     return;
   }
@@ -311,10 +330,9 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) k_slab(SlabShape f, SlabArgs 
         }
       }
   }
-  bool ok = true;
   if (KEEP) {
-    __syncthreads();  // the barrier is initialised
-    ok = umma::mbar_wait_bounded(&bar, 0u);
+    __syncthreads();  // the barriers are initialised
+    slab_operands(bar, lim, stall, &q.ctrl->umma_err);
   }
   cl.sync();  // the slab is loaded; every CTA runs before any remote write
   double s0 = 0.0, s1 = 0.0;
@@ -397,7 +415,8 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) k_slab(SlabShape f, SlabArgs 
     __shared__ int last;
     block_sum2<SLAB_THREADS>(s0, s1, red);
     if (tid == 0) {
-      q.partials[2 * blockIdx.x] = ok ? s0 : nan("");
+      // an expired wait of this kernel's CTA or of an earlier kernel of the step
+      q.partials[2 * blockIdx.x] = *(volatile int*)&q.ctrl->umma_err ? nan("") : s0;
       q.partials[2 * blockIdx.x + 1] = s1;
       __threadfence();
       last = atomicAdd(&q.ctrl->tickets, 1u) == gridDim.x - 1;
