@@ -297,10 +297,12 @@ int sgh_box_window(sgh_plan* plan, int32_t* i0, void* stream);
 #define SGH_PICARD_HISTORY_MAX 4096
 int sgh_picard_history(sgh_plan* plan, double* out, int32_t cap, int32_t* n_iter, void* stream);
 
-/* Bound of the data waits of a plan's slab kernels (the fused volume form): at
+/* Bound of the data waits of a plan's slab kernels (the fused volume form) and
+ * of its face-space cluster kernel: at
  * most `polls` mbarrier polls (0 = the default, 2^22) before the kernel records
- * the error, waits for its copies in flight (with the default bound) and goes
- * on; the step's Picard loop then ends and the step reports SGH_STEP_TC_TIMEOUT,
+ * the error and waits for its copies in flight (with the default bound). The
+ * step's Picard loop then ends (the cluster kernel writes no results at all) and
+ * the step reports SGH_STEP_TC_TIMEOUT,
  * as do later ones until the plan is bound again. stall_test = 1 makes every
  * such wait run out (needs polls > 0), so that a test can drive the error path
  * without a fault; 0 for normal stepping. No reference counterpart.
@@ -401,14 +403,15 @@ int sgh_batch_status(const sgh_batch* batch, sgh_batch_slot_info* out, void* str
 /* Device pointer / size of a slot buffer: SGH_BUF_MODES, SGH_BUF_K, SGH_BUF_KK
  * (element type FP64 or FP32 by precision), SGH_BUF_Q_EVAP_OLD, SGH_BUF_SURFACE (FP64). */
 int sgh_batch_buffer(const sgh_batch* batch, int32_t slot, int32_t which, void** ptr, uint64_t* bytes);
-/* *err = nonzero once a tensor-core wait of a mixed-precision batch expired
- * (the affected face pass wrote no results). Synchronises the stream. */
+/* *err = nonzero once a bounded wait of the batch's face or volume kernels
+ * expired (the affected face pass, or the whole face step of a slot that runs
+ * in a cluster, wrote no results; such a slot's step ends SGH_STEP_NONFINITE). Synchronises the stream. */
 int sgh_batch_error(const sgh_batch* batch, int32_t* err, void* stream);
-/* Bound of the tensor-core data waits of the batch's face transforms: at most
- * `polls` mbarrier polls (0 = the default, 2^22) before the CTA records the
- * error flag, waits for its copies and MMAs in flight (always with the
+/* Bound of the data waits of the batch's face transforms and cluster kernels:
+ * at most `polls` mbarrier polls (0 = the default, 2^22) before the CTA records
+ * the error flag, waits for its copies and MMAs in flight (always with the
  * default bound), frees its tensor memory and returns without results.
- * stall_test = 1 makes every face-transform CTA first wait, with that bound,
+ * stall_test = 1 makes every such CTA first wait, with that bound,
  * on a barrier that nothing completes -- a wait that can only run out -- so a
  * test can drive the error path without a fault (needs polls > 0); 0 for
  * normal stepping. No reference counterpart: the reference has no bounded

@@ -256,14 +256,14 @@ class BatchSolver:
         self.stream.synchronize()
 
     def tensor_core_error(self) -> int:
-        """Nonzero once a tensor-core wait expired in a mixed-precision face pass."""
+        """Nonzero once a bounded wait of a face or volume kernel expired."""
         e = C.c_int32()
         _lib.check("sgh_batch_error", _lib.lib().sgh_batch_error(self._h, C.byref(e), self._s()))
         return e.value
 
     def set_wait_limit(self, polls: int = 0, stall_test: bool = False) -> None:
-        """Bound the tensor-core data waits to ``polls`` polls (0: the default);
-        ``stall_test`` makes the face transforms wait on a barrier nothing
+        """Bound the data waits to ``polls`` polls (0: the default); ``stall_test``
+        makes the face transforms and cluster kernels wait on a barrier nothing
         completes, so the bounded-wait error path runs (tests only)."""
         _lib.check("sgh_batch_set_wait_limit", _lib.lib().sgh_batch_set_wait_limit(
             self._h, int(polls), 1 if stall_test else 0, self._s()))

@@ -791,7 +791,8 @@ k_face_run(const DevParams* __restrict__ P, Ctrl* ctrl, fold::FaceShape f, fold:
   J.ly = L.y;
   J.shift_x = laser_shift(L.vx, P->dt, P->dx, f32);
   J.shift_y = laser_shift(L.vy, P->dt, P->dy, f32);
-  const bool ok = fold::face_operands(f, J, fr_sh, bar, umma::WAIT_LIMIT, false, &ctrl->umma_err);
+  const unsigned lim = ctrl->wait_limit ? ctrl->wait_limit : umma::WAIT_LIMIT;
+  const bool ok = fold::face_operands(f, J, fr_sh, bar, lim, ctrl->stall_test != 0, &ctrl->umma_err);
   const fold::FaceResult r = fold::face_step<double, KEEPM>(f, J, fr_sh, !ok);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     sgh_step_out o;

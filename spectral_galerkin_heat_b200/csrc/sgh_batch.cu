@@ -97,12 +97,12 @@ struct BState {
 
 struct BGlobal {
   int steps_left;
-  int umma_err;     // nonzero once a tensor-core wait expired
+  int umma_err;     // nonzero once a bounded data wait expired
   int picard_any;   // some slot is still iterating (read by the eager step)
   unsigned slots_done;   // slots finished in the current kb_relax launch (back to 0 after it)
   int n_iter_slots;      // slots iterating in the current Picard iteration
-  unsigned wait_limit;   // polls of the tensor-core data waits (0: umma::WAIT_LIMIT)
-  int stall_test;        // 1: every face y-pass CTA first waits on a barrier nothing completes
+  unsigned wait_limit;   // polls of the data waits (0: umma::WAIT_LIMIT)
+  int stall_test;        // 1: face y-pass and cluster CTAs first wait on a barrier nothing completes
   int pad;
 };
 

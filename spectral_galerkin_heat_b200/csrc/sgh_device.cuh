@@ -67,7 +67,7 @@ struct Ctrl {
   int hist_cap;
   unsigned tickets;  // CTAs of the current relaxation done (back to 0 after it)
   int umma_err;  // a bounded wait of one of the plan's kernels ran out
-  unsigned wait_limit;  // polls of the slab kernels' waits (0: umma::WAIT_LIMIT)
+  unsigned wait_limit;  // polls of the slab and cluster kernels' waits (0: umma::WAIT_LIMIT)
   int stall_test;       // 1: they first wait on a barrier that nothing completes
 };
 

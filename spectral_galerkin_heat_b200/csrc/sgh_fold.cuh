@@ -344,16 +344,19 @@ __device__ __forceinline__ void copy_async(W* dst, const W* src) {
 }
 
 // All threads of all CTAs of the cluster. The result is complete on rank 0,
-// thread 0. bad: this CTA's operands are invalid (an expired wait): its
-// partials become NaN and the step ends non-finite. KEEPM: the packed matrices
+// thread 0. bad: this CTA's operands are invalid (an expired wait): the cluster then
+// writes no results (q_evap, sigma and the surface stay as they were) and the step
+// ends non-finite. KEEPM: the packed matrices
 // are in shared memory (FACE_M), addressed as such.
 template <class W, bool KEEPM>
 __device__ FaceResult face_step(const FaceShape& f, const FaceJob<W>& J, double* sm, bool bad) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
+  __shared__ int sbad;
   const int n = f.n, rank = (int)cl.block_rank();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int NW = blockDim.x >> 5;
+  if (tid == 0) sbad = bad ? 1 : 0;
   auto sync_all = [&] {  // one CTA: a block barrier is a tenth of a cluster barrier
     if (n > 1) cl.sync();
     else __syncthreads();
@@ -428,6 +431,21 @@ __device__ FaceResult face_step(const FaceShape& f, const FaceJob<W>& J, double*
   n1 = warp_sum(n1);
   sync_all();  // also: every CTA of the cluster runs before any remote write
 
+  FaceResult res;
+  res.iter = -1;
+  res.status = SGH_STEP_CAPPED;
+  res.rel = nan("");
+  // every warp reads every CTA's flag, so all leave here together or none does; the
+  // second barrier keeps each CTA's shared memory until the others have read it
+  if (__any_sync(0xffffffffu, lane < n && *cl.map_shared_rank(&sbad, lane < n ? lane : 0) != 0)) {
+    cp_async_wait<0>();
+    sync_all();
+    res.iter = 0;
+    res.status = SGH_STEP_NONFINITE;
+    res.tmax = res.qsum = nan("");
+    return res;
+  }
+
   // transposes: row domain -> the column owners' xc, column domain -> the row owners' xr
   auto to_columns = [&](int p, int v, double x0, double x1) {
     const int dst = (int)(((float)p + 0.5f) * rC);
@@ -461,10 +479,6 @@ __device__ FaceResult face_step(const FaceShape& f, const FaceJob<W>& J, double*
   };
   const int hx = half_up(nx), VT = (nx + 7) / 8, PT = (ny + 7) / 8, vt_n = (nc + 7) / 8;
 
-  FaceResult res;
-  res.iter = -1;
-  res.status = SGH_STEP_CAPPED;
-  res.rel = nan("");
   double mx = -INFINITY;
   for (;;) {
     // q_net -> its 2-D transform, first along rows, then along columns
@@ -501,7 +515,7 @@ __device__ FaceResult face_step(const FaceShape& f, const FaceJob<W>& J, double*
         o2 = warp_sum(o2);
         if (lane < n)
           *reinterpret_cast<double2*>(cl.map_shared_rank(part, lane) + 2 * (pt * VT + c0 / 8 + vt)) =
-              make_double2(bad ? nan("") : r2, o2);
+              make_double2(r2, o2);
       }
     }
     ++res.iter;
@@ -625,8 +639,9 @@ __device__ bool face_operands(const FaceShape& f, const FaceJob<W>& J, double* s
     ok = ok && mbar_wait_bounded(&bar[0], 0u, lim);
     if (!ok) mbar_wait_bounded(&bar[0], 0u, WAIT_LIMIT);
   }
+  ok = __syncthreads_and(ok ? 1 : 0) != 0;
   if (!ok && threadIdx.x == 0 && err) atomicExch(err, 1);
-  return __syncthreads_and(ok ? 1 : 0) != 0;
+  return ok;
 }
 
 // Cluster launch of a face kernel; `pdl`: programmatic stream serialisation

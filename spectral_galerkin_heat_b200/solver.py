@@ -394,9 +394,10 @@ class B200SpectralSolver(HeatSolver):
         return hist
 
     def set_wait_limit(self, polls: int = 0, stall_test: bool = False) -> None:
-        """Bound the data waits of the fused volume form to ``polls`` polls (0:
-        the default); ``stall_test`` makes them wait on a barrier nothing
-        completes, so that the error path runs (tests only)."""
+        """Bound the data waits of the fused volume form and of the face-space
+        cluster kernel to ``polls`` polls (0: the default); ``stall_test`` makes
+        them wait on a barrier nothing completes, so that the error path runs
+        (tests only)."""
         self._require()
         _lib.check("sgh_plan_set_wait_limit", _lib.lib().sgh_plan_set_wait_limit(
             self._plan, int(polls), 1 if stall_test else 0, C.c_void_p(self.state.stream.cuda_stream)))
