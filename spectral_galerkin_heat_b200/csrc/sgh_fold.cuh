@@ -467,11 +467,13 @@ __device__ FaceResult face_step(const FaceShape& f, const FaceJob<W>& J, double*
   auto keep_col = [&](int p, int v, double x0, double x1) {
     *reinterpret_cast<double2*>(&xt[p * ldc + v]) = make_double2(x0, x1);
   };
-  // two vector tiles per matrix fragment where that still leaves every warp a task
+  // two vector tiles per matrix fragment where there are two and that still leaves every
+  // warp a task (with two for a share of one tile, half the products were
+  // dropped: a 512 x 64 face, 12 iterations, 780 us a step, now 540)
   auto pass = [&](auto kind, const double* P, int N, const double* X, int sk, int sv, int nvec, const auto& out) {
     constexpr int KIND = decltype(kind)::value;
     if (nvec <= 0) return;
-    if (mtiles(N) * ((nvec + 15) / 16) >= NW) fold_pass<KIND, 2>(P, N, X, sk, sv, nvec, warp, NW, out);
+    if (nvec > 8 && mtiles(N) * ((nvec + 15) / 16) >= NW) fold_pass<KIND, 2>(P, N, X, sk, sv, nvec, warp, NW, out);
     else fold_pass<KIND, 1>(P, N, X, sk, sv, nvec, warp, NW, out);
   };
   auto weight = [&](int which, const W* src, int li, size_t gi) -> double {

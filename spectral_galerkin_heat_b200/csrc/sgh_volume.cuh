@@ -171,11 +171,12 @@ __device__ __forceinline__ void slab_pass(const double* P, int N, const double* 
   }
 }
 
-// Vector tiles per task: two where that still leaves eight tasks.
+// Vector tiles per task: two where there are two and that still leaves eight tasks
+// (512 x 128 x 32, an iteration: 744 us with two for shares of one tile, 576 now).
 template <bool FWD, class O>
 __device__ __forceinline__ void slab_run(const double* P, int N, const double* X, int sk, int sv, int nvec, int warp,
                                          int nwarps, const O& out) {
-  if (mtiles(N) * ((nvec + 15) / 16) >= 8) slab_pass<FWD, 2, true>(P, N, X, sk, sv, nvec, warp, nwarps, out);
+  if (nvec > 8 && mtiles(N) * ((nvec + 15) / 16) >= 8) slab_pass<FWD, 2, true>(P, N, X, sk, sv, nvec, warp, nwarps, out);
   else slab_pass<FWD, 1, true>(P, N, X, sk, sv, nvec, warp, nwarps, out);
 }
 
