@@ -244,13 +244,14 @@ struct SlabArgs {
 
 // Waits for the packed matrices' copies on bar[0], at most lim polls a thread. A
 // thread whose wait ran out (or, with `stall`, that first waited on bar[1], which
-// nothing completes) records it in *err and waits for the copies with the full
-// bound, so that none outlives the CTA.
-__device__ __forceinline__ void slab_operands(uint64_t* bar, unsigned lim, bool stall, int* err) {
+// nothing completes) records it in *err and *expired and waits for the copies with
+// the full bound, so that none outlives the CTA.
+__device__ __forceinline__ void slab_operands(uint64_t* bar, unsigned lim, bool stall, int* err, int* expired) {
   bool ok = !stall || umma::mbar_wait_bounded(&bar[1], 0u, lim);
   ok = ok && umma::mbar_wait_bounded(&bar[0], 0u, lim);
   if (!ok) {
     atomicExch(err, 1);
+    *expired = 1;
     umma::mbar_wait_bounded(&bar[0], 0u, umma::WAIT_LIMIT);
   }
 }
@@ -265,6 +266,7 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) k_slab(SlabShape f, SlabArgs 
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ __align__(128) double sl_sh[];
   __shared__ uint64_t bar[2];
+  __shared__ int expired;  // a wait of this CTA ran out
   __shared__ double red[2 * (SLAB_THREADS / 32)];
   constexpr int NW = SLAB_THREADS / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -283,6 +285,7 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) k_slab(SlabShape f, SlabArgs 
   const double* pyi = KEEP ? sl_sh + f.o_m + nyp + 2 * nxp : q.pyi;
   // The packed matrices never change: their copies start before the wait for
   // the previous kernel.
+  if (tid == 0) expired = 0;
   if (KEEP && tid == 0) {
     double* o = sl_sh + f.o_m;
     umma::mbar_init(&bar[0], 1);
@@ -295,12 +298,13 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) k_slab(SlabShape f, SlabArgs 
     umma::bulk_g2s(o + nyp + 2 * nxp, q.pyi, 8 * nyp, &bar[0]);
   }
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
-  const unsigned lim = KEEP && q.ctrl->wait_limit ? q.ctrl->wait_limit : umma::WAIT_LIMIT;
-  const bool stall = KEEP && q.ctrl->stall_test != 0;
+  // read here, used far below: the flag of the step's earlier kernels, the waits' bound
+  const int err0 = q.ctrl->umma_err, stall = q.ctrl->stall_test;
+  const unsigned limit = q.ctrl->wait_limit;
   if (MODE == SLAB_QM && q.ctrl->iter <= 0) {  // the same for every CTA
     if (KEEP) {
       __syncthreads();
-      slab_operands(bar, lim, stall, &q.ctrl->umma_err);  // no copy outlives the CTA
+      slab_operands(bar, limit ? limit : umma::WAIT_LIMIT, stall != 0, &q.ctrl->umma_err, &expired);  // no copy outlives the CTA
     }
     return;
   }
@@ -333,7 +337,7 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) k_slab(SlabShape f, SlabArgs 
   }
   if (KEEP) {
     __syncthreads();  // the barriers are initialised
-    slab_operands(bar, lim, stall, &q.ctrl->umma_err);
+    slab_operands(bar, limit ? limit : umma::WAIT_LIMIT, stall != 0, &q.ctrl->umma_err, &expired);
   }
   cl.sync();  // the slab is loaded; every CTA runs before any remote write
   double s0 = 0.0, s1 = 0.0;
@@ -416,8 +420,7 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) k_slab(SlabShape f, SlabArgs 
     __shared__ int last;
     block_sum2<SLAB_THREADS>(s0, s1, red);
     if (tid == 0) {
-      // an expired wait of this kernel's CTA or of an earlier kernel of the step
-      q.partials[2 * blockIdx.x] = *(volatile int*)&q.ctrl->umma_err ? nan("") : s0;
+      q.partials[2 * blockIdx.x] = err0 || expired ? nan("") : s0;
       q.partials[2 * blockIdx.x + 1] = s1;
       __threadfence();
       last = atomicAdd(&q.ctrl->tickets, 1u) == gridDim.x - 1;
