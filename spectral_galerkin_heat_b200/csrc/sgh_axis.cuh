@@ -24,6 +24,7 @@
 #include <utility>
 
 #include "sgh_device.cuh"
+#include "sgh_limits.h"
 #include "sgh_umma.cuh"
 
 namespace sgh {
@@ -835,11 +836,7 @@ template <bool CONTIG, int NC, class Epi>
 inline void launch_axis_umma_nc(const double* X, const double* Mat, const char* pair, int Nout, int N, int A,
                                 int B, const Epi& epi, dim3 grid, cudaStream_t st) {
   constexpr int bytes = axu_smem_bytes<NC>();
-  static const bool attr = [] {
-    cudaFuncSetAttribute(k_axis_umma<CONTIG, NC, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    return true;
-  }();
-  (void)attr;
+  (void)kernel_limits(reinterpret_cast<const void*>(k_axis_umma<CONTIG, NC, Epi>), bytes);
   launch_pdl(k_axis_umma<CONTIG, NC, Epi>, grid, AXU_THREADS, bytes, st, X, Mat, pair, Nout, N, A, B, epi,
              g_umma_err);
 }
@@ -943,16 +940,12 @@ inline int axis_blocks(int Nout, int A, int B) {
 }
 
 // Dynamic shared memory of the tensor-core kernel, raised past the 48 KB
-// default once per instantiation.
+// default once per instantiation and device.
 template <bool CONTIG, int BM, int BN, class Epi>
 inline void launch_axis_mma(const double* X, const double* Mat, int Nout, int N, int A, int B, const Epi& epi,
                             dim3 grid, cudaStream_t st) {
   constexpr int bytes = axm_smem_bytes<CONTIG, BM, BN>();
-  static const bool attr = [] {
-    cudaFuncSetAttribute(k_axis_mma<CONTIG, BM, BN, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    return true;
-  }();
-  (void)attr;
+  (void)kernel_limits(reinterpret_cast<const void*>(k_axis_mma<CONTIG, BM, BN, Epi>), bytes);
   launch_pdl(k_axis_mma<CONTIG, BM, BN, Epi>, grid, AX_THREADS, bytes, st, X, Mat, Nout, N, A, B, epi);
 }
 

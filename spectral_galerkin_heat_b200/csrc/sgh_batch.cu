@@ -40,6 +40,7 @@
 #include "sgh_axis.cuh"
 #include "sgh_device.cuh"
 #include "sgh_fold.cuh"
+#include "sgh_limits.h"
 #include "sgh_umma.cuh"
 
 namespace sgh {
@@ -1726,8 +1727,8 @@ template <bool INV, bool SKIP, int KIND, class EpiF>
 void face2d(sgh_batch* B, cudaStream_t s, const double* in, const EpiF& ef, const F2Args& fa, double* part) {
   const BView v = B->view();
   if (B->precision == SGH_PRECISION_MIXED) {
-    (void)cudaFuncSetAttribute(kb_fx<INV, SKIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, f2::SMEM);
-    (void)cudaFuncSetAttribute(kb_fy<INV, SKIP, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, f2::SMEM);
+    (void)kernel_limits(reinterpret_cast<const void*>(kb_fx<INV, SKIP>), f2::SMEM);
+    (void)kernel_limits(reinterpret_cast<const void*>(kb_fy<INV, SKIP, KIND>), f2::SMEM);
     kb_fx<INV, SKIP><<<B->tot_utile, f2::THREADS, f2::SMEM, s>>>(v);
     kb_fy<INV, SKIP, KIND><<<B->tot_utile, f2::THREADS, f2::SMEM, s>>>(v, fa, part);
     g_blaunch += 2;

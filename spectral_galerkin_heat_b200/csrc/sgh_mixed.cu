@@ -10,6 +10,7 @@
 
 #include "sgh_b200.h"
 #include "sgh_device.cuh"
+#include "sgh_limits.h"
 #include "sgh_umma.cuh"
 
 namespace sgh {
@@ -61,7 +62,7 @@ template <int NT, int PASS>
 int launch_pass(const double* in, double* out, const double* Mx, const double* My, int ny, int nx, int* err,
                 cudaStream_t s) {
   const int smem = umma::smem_bytes(NT);
-  cudaError_t e = cudaFuncSetAttribute(k_dct2_bf16x3<NT, PASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = kernel_limits(reinterpret_cast<const void*>(k_dct2_bf16x3<NT, PASS>), smem);
   if (e != cudaSuccess) return set_error(SGH_ERR_CUDA, cudaGetErrorString(e));
   dim3 grid((nx + NT - 1) / NT, (ny + umma::TM - 1) / umma::TM);
   k_dct2_bf16x3<NT, PASS><<<grid, umma::THREADS, smem, s>>>(in, out, Mx, My, ny, nx, err);

@@ -28,6 +28,7 @@
 #include <algorithm>
 
 #include "sgh_axis.cuh"
+#include "sgh_limits.h"
 
 namespace sgh {
 namespace sym {
@@ -295,11 +296,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_sym(Args q) {
 template <bool CONTIG, bool FWD>
 inline void launch_one(const Args& q, cudaStream_t st) {
   using L = Lay<CONTIG, FWD>;
-  static const bool attr = [] {
-    cudaFuncSetAttribute(k_sym<CONTIG, FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES);
-    return true;
-  }();
-  (void)attr;
+  (void)kernel_limits(reinterpret_cast<const void*>(k_sym<CONTIG, FWD>), L::BYTES);
   const int H = FWD ? (q.Nout + 1) / 2 : std::max(1, q.Nout / 2);
   const dim3 grid((unsigned)(((long long)q.A * q.B + BC - 1) / BC), (unsigned)((H + BJ - 1) / BJ));
   launch_pdl(k_sym<CONTIG, FWD>, grid, THREADS, L::BYTES, st, q);

@@ -79,3 +79,11 @@ def test_limits_only_grow_per_kernel_and_device(tmp_path):
                    check=True)
     out = subprocess.run([str(exe)], capture_output=True, text=True)
     assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout
+
+
+def test_no_kernel_sets_its_limits_any_other_way():
+    """A limit raised once per process would hold on the first device only."""
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".cuh", ".h")) and name != "sgh_limits.h":
+            text = open(os.path.join(CSRC, name)).read()
+            assert "cudaFuncSetAttribute" not in text, name
