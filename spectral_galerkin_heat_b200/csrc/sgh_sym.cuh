@@ -71,9 +71,11 @@ __global__ void __launch_bounds__(THREADS, 2) k_sym(Args q) {
   // output pairs (the middle output of an odd inverse form is not one), slices a
   // forward pass keeps
   const int H = FWD ? (Nout + 1) / 2 : Nout / 2, h = (N + 1) / 2;
-  // The middle output contracts the even slices only. It is summed by the CUDA
+  // The middle output has zero weights on the odd slices. It is summed by the CUDA
   // cores of the last row of CTAs from the staged slices: as one more pair it would
-  // cost a tile of 32 (N / 2 + 1 pairs of a node matrix: 3 tiles of 32 for 64).
+  // cost a tile of 32 (N / 2 + 1 pairs of a node matrix: 3 tiles of 32 for 64). The
+  // odd slices are added with their zeros, so that a NaN or an infinity among them
+  // reaches this output as it reaches every other.
   const bool mid = !FWD && (Nout & 1) && blockIdx.y == gridDim.y - 1;
   double msum = 0.0;
   const int c0 = blockIdx.x * BC, j0 = blockIdx.y * BJ;
@@ -199,7 +201,10 @@ __global__ void __launch_bounds__(THREADS, 2) k_sym(Args q) {
 #pragma unroll
       for (int i = 0; i < KP * BC / THREADS; ++i) {
         const int s = 2 * (tid / BC + (THREADS / BC) * i), n = 2 * KP * ch + s;
+        // the odd slice beyond the length is staged as zero
+        const double x1 = CONTIG ? Xs[col * L::LDX + s + 1] : Xs[(s + 1) * L::LDX + col];
         if (n < N) msum = fma(__ldg(q.Mat + (size_t)(Nout / 2) * N + n), CONTIG ? Xs[col * L::LDX + s] : Xs[s * L::LDX + col], msum);
+        msum = fma(0.0, x1, msum);
       }
     }
 #pragma unroll
