@@ -2301,14 +2301,9 @@ int sgh_box_project(sgh_plan* p, const double* field_box, double* modes, void* s
 
 namespace {
 // Whether a pass of sgh_dctn takes the halved contraction (sgh_sym.cuh): axes
-// below one tile, and long axes of few columns (under 40 of its CTAs), stay on
-// the small tiles of launch_axis. A pair of transforms, both ways measured: 96 x
-// 60 x 100 86 -> 66 us, 50 x 100 x 200 168 -> 117, 100 x 128 x 256 312 -> 250, 1-D
-// 1000 97 -> 90; 256 x 512, with 32 CTAs in its x-pass, 77 -> 80 halved.
-bool sym_pass(int N, long ncol) {
-  const long ctas = ((ncol + sym::BC - 1) / sym::BC) * (((N + 1) / 2 + sym::BJ - 1) / sym::BJ);
-  return N >= 16 && (ctas >= 40 || N <= 128 || ncol == 1);
-}
+// below one tile stay on the small tiles of launch_axis, and long axes of few
+// columns where sym::fills() says so.
+bool sym_pass(int N, long ncol) { return N >= 16 && (ncol == 1 || sym::fills(N, N, ncol)); }
 
 struct DctnLayout {
   int n[3] = {1, 1, 1};   // (n0, n1, n2), n2 fastest; unused leading axes are 1

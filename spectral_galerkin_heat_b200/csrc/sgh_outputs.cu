@@ -159,6 +159,27 @@ int sgh_nodal_workspace_bytes(int32_t nx, int32_t ny, int32_t nz, uint64_t* byte
   return SGH_OK;
 }
 
+// Result of a full contraction at the strides of a halved one: output (a, k, b) of
+// a pass over [A][Nout][B] at a * sa + k * sk + b.
+struct EpiStrided {
+  static constexpr int kReduce = 0;
+  double* out;
+  int Nout, B;
+  long long sa, sk;
+  double* partials;
+  __device__ __forceinline__ void operator()(int i, int, int, double v, Red&) const {
+    const int t = i / B, b = i - t * B, a = t / Nout, k = t - a * Nout;
+    out[a * sa + k * sk + b] = v;
+  }
+};
+
+// One pass of the node field: halved where that fills the GPU (sym::fills).
+static void node_pass(const double* X, const double* B, double* out, int N, int A, int cols, long long sa,
+                      long long sk, bool kfast, cudaStream_t s) {
+  if (sym::fills(N + 1, N, (long long)A * cols)) sym::launch(3, X, B, out, N + 1, N, A, cols, sa, sk, kfast, s);
+  else launch_axis(X, B, N + 1, N, A, cols, EpiStrided{out, N + 1, cols, sa, sk, nullptr}, s);
+}
+
 // The passes run z, y, x: every intermediate then has an even contiguous length
 // where the modes have one (16-byte copies), and the last pass can write either
 // axis order. B[N - j][m] = (-1)^m B[j][m]: the passes are halved (sgh_sym.cuh).
@@ -184,13 +205,13 @@ static int nodal(int32_t nx, int32_t ny, int32_t nz, double Lx, double Ly, doubl
   // (ny+1, nz+1, nx) for the transposed output; x: -> (nz+1, ny+1, nx+1), or from the
   // columns (y, z) straight into (nx+1, ny+1, nz+1)
   const long long S = (long long)nx * ny, X = nx, cols = (long long)(ny + 1) * (nz + 1);
-  sym::launch(3, modes, Bz, out, nz + 1, nz, 1, (int)S, 0, S, false, s);
+  node_pass(modes, Bz, out, nz, 1, (int)S, 0, S, false, s);
   if (xyz) {
-    sym::launch(3, out, By, tmp, ny + 1, ny, nz + 1, nx, X, (nz + 1) * X, false, s);
-    sym::launch(3, tmp, Bx, out, nx + 1, nx, (int)cols, 1, 1, cols, false, s);
+    node_pass(out, By, tmp, ny, nz + 1, nx, X, (nz + 1) * X, false, s);
+    node_pass(tmp, Bx, out, nx, (int)cols, 1, 1, cols, false, s);
   } else {
-    sym::launch(3, out, By, tmp, ny + 1, ny, nz + 1, nx, (ny + 1) * X, X, false, s);
-    sym::launch(3, tmp, Bx, out, nx + 1, nx, (int)cols, 1, X + 1, 1, true, s);
+    node_pass(out, By, tmp, ny, nz + 1, nx, (ny + 1) * X, X, false, s);
+    node_pass(tmp, Bx, out, nx, (int)cols, 1, X + 1, 1, true, s);
   }
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(SGH_ERR_CUDA, cudaGetErrorString(e));

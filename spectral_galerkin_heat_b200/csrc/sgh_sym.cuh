@@ -296,6 +296,19 @@ __global__ void __launch_bounds__(THREADS, 2) k_sym(Args q) {
   }
 }
 
+// Whether a pass has enough CTAs for k_sym: past 128 its CTAs' chains of chunks are
+// longer than those of launch_axis's smaller tiles, and under about 100 CTAs they
+// leave SMs idle besides. A pair of transforms with every pass on the full
+// contraction, with k_sym from 40 CTAs, with k_sym from 100: 512 x 512 (64 CTAs a
+// pass) 96, 101, 82 us; 400 x 400 (49) 82, 87, 66; 20 x 600 x 20 (70) 89, 94, 77;
+// 600 x 600 (100) 156, 119, 119; 30 x 600 x 20 (100) 115, 95, 95. Node field of 600 x
+// 20 x 20 (70 CTAs in its x-pass) 48, 50, 44 us, of 1000 x 10 x 10 (32) 61, 81, 69.
+constexpr int MIN_CTAS = 100;
+inline bool fills(int Nout, int N, long long ncol) {
+  const long long ctas = ((ncol + BC - 1) / BC) * ((std::max(1, (Nout + 1) / 2) + BJ - 1) / BJ);
+  return N <= 128 || ctas >= MIN_CTAS;
+}
+
 // One pass; kind: 2 forward (DCT-II matrix), 3 inverse form. Output element (a, k, b)
 // at a * sa + k * sk + b; kfast when that is contiguous along k.
 template <bool CONTIG, bool FWD>
