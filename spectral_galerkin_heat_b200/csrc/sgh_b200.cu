@@ -1585,12 +1585,33 @@ int fused_slab(const sgh_plan* p) {
 }
 
 // Cluster size of the face-space step, or 0 for the multi-kernel form
-// (convection, reduced precision, faces too large for a cluster).
+// (convection, reduced precision, faces too large for a cluster, and those whose
+// passes on the cluster's few SMs take longer than the chip-wide ones and their
+// launches). Measured over 42 faces, us a step, one pass per axis / cluster:
+//   face        chain   one forcing pass    12 iterations
+//   256 x 128      48      110 /  85          458 / 298
+//   384 x 96      120      119 / 104          602 / 449
+//   256 x 224     120      122 / 122          614 / 542
+//   256 x 256     128      125 / 132          636 / 584
+//   400 x 128     132      125 / 121          643 / 556
+//   512 x 64      140      128 / 118          658 / 540
+//   288 x 144     144      115 / 129          573 / 600
+//   320 x 160     160      121 / 141          611 / 641
+//   300 x 200     205      126 / 166          640 / 800
+//   16 x 400      104      106 / 111          532 / 528
+//   16 x 600      270      136 / 164          722 / 854
+// With one forcing pass per step the chip-wide passes of small faces are the
+// shorter ones (hence the bound by the size), and from 4096 cells a CTA the laser
+// flux, which the chip-wide form spreads over every SM, decides.
 int face_cluster(const sgh_plan* p) {
   const DevParams& h = p->hp;
   if (!p->face_space || h.has_top_conv || h.has_bottom_conv) return 0;
   if (p->cfg.precision != SGH_PRECISION_FP64) return 0;
-  return fold::cluster_size<double>(h.nx, h.ny);
+  const int n = fold::cluster_size<double>(h.nx, h.ny);
+  if (!n) return 0;
+  const bool once = p->cfg.max_iter <= 1;
+  if (once && h.S >= 4096 * n) return 0;
+  return fold::face_chain(h.nx, h.ny, n) <= (once ? std::min(140, 84 + h.S / 340) : 140) ? n : 0;
 }
 
 // Adds a conditional node of the given type to the graph being captured on

@@ -300,6 +300,19 @@ __host__ inline int cluster_size_crowded(int nx, int ny) {
     if ((long)nx * ny <= FACE_SHARE_CROWDED * n && face_shape<W>(nx, ny, n).bytes <= FACE_SMEM_MAX - 512) return n;
   return cluster_size<W>(nx, ny);
 }
+// Estimated length of a Picard iteration's four passes on a cluster, in slice steps
+// of its longest chain of tasks: 16 warps a CTA, a task is one 16-row fragment row
+// of one half over the slices of one vector tile (see fold_pass). A long axis
+// gives few CTAs many fragment rows, shares of several tiles give many tasks.
+inline int face_chain(int nx, int ny, int n) {
+  const int R = ((ny + 7) / 8 + n - 1) / n, C = ((nx + 7) / 8 + n - 1) / n;  // vector tiles a CTA
+  const auto pass = [](int N, int tiles, int halves) {
+    const bool two = tiles > 1 && mtiles(N) * ((tiles + 1) / 2) >= 16;
+    const int tasks = halves * mtiles(N) * (two ? (tiles + 1) / 2 : tiles);
+    return (tasks + 15) / 16 * ksteps(N) * (two ? 2 : 1);
+  };
+  return 2 * pass(nx, R, 2) + pass(ny, C, 2) + 2 * pass(ny, C, 1);
+}
 // Threads of a face kernel: eight warps cover the tasks of a small share
 // (64 x 32 on 4 CTAs: 407 us with 256 or 512 threads, 437 with 128), larger
 // ones want sixteen (256 x 128: 884 us with 256, 749 with 512, at 8 CTAs).

@@ -1,0 +1,51 @@
+"""Which form a single-instance plan takes, on both sides of the rules that
+choose it, and that either form gives the oracle's steps to 1e-10 (the bound of
+every FP64 form). Faces: one cluster, or one pass per axis where the cluster's
+few SMs would take longer."""
+import ctypes as C
+
+import pytest
+
+from conftest import make_context, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _counts(s):
+    from spectral_galerkin_heat_b200 import _lib
+    a, b, c = C.c_int32(), C.c_int32(), C.c_int32()
+    _lib.check("launch_counts", _lib.lib().sgh_plan_launch_counts(s._plan, C.byref(a), C.byref(b), C.byref(c)))
+    return a.value, b.value, c.value
+
+
+def _against_oracle(ctx, steps=2, **kw):
+    from oracle.sgh_oracle import OracleSolver
+    from spectral_galerkin_heat_b200 import B200SpectralSolver
+    o = OracleSolver(ctx)
+    o.initialize()
+    s = B200SpectralSolver(None, ctx, **kw)
+    s.initialize()
+    dt = ctx.num.dt
+    for k in range(steps):
+        _, mo = o.step(k * dt, dt)
+        _, m = s.step(k * dt, dt)
+        assert m["n_evap_iter"] == mo["n_evap_iter"]
+    counts, err = _counts(s), rel_l2(s.state.a.cpu().numpy(), o.a)
+    s.finalize()
+    return counts, err
+
+
+@pytest.mark.parametrize("nx,ny,cap,cluster", [
+    (64, 32, 1, True), (512, 64, 1, True), (512, 64, 6, True), (256, 256, 1, False), (256, 256, 6, True),
+    (16, 400, 1, False), (16, 400, 6, True), (288, 144, 6, False), (300, 200, 1, False), (1000, 16, 6, False)])
+def test_face_form(nx, ny, cap, cluster):
+    from spectral_galerkin_heat_b200 import workloads
+    from spectral_galerkin_heat_b200.laser import StraightTrack
+    size = (nx * 3e-5, ny * 3e-5, 2e-4)
+    cfg, _ = workloads.straight_track(nx=nx, ny=ny, nz=4, steps=3, size=size)
+    if cap > 1:
+        cfg["simulation"].update({"max_picard_iter": cap, "picard_omega": 0.1, "picard_tol": 1e-4})
+    ctx = make_context(cfg, StraightTrack(0.4 * size[0], 0.45 * size[1], 0.8, 0.3, 120.0))
+    counts, err = _against_oracle(ctx)
+    assert (counts[1] == 0) == cluster   # a cluster iterates inside its one kernel
+    assert err < 1e-10
