@@ -1567,9 +1567,11 @@ bool phase_branches(const sgh_config& c) {
 }
 
 // CTAs per slab of the fused volume form, or 0 for one pass per axis: grid
-// mode in FP64, or in mixed precision (FP64 contractions there are more exact
-// than the split-BF16 ones and, fused, faster: 128 x 64 x 32, 3 steps, 14.3 -> 7.7
-// ms). One pass per axis remains for slabs that fit no cluster, for FP32 plans,
+// mode in FP64 where it is the faster of the two (vol::slab_wins), and in mixed
+// precision (FP64 contractions there are more exact than the split-BF16 ones and,
+// fused, faster at every size measured: 32 x 16 x 8 64 -> 40 us an iteration, 128 x
+// 64 x 32 105 -> 59, 512 x 256 x 64 3418 -> 2095). One pass per axis remains for
+// slabs that fit no cluster, for FP32 plans,
 // and for properties that jump between the phases: their fixed-point map need
 // not contract in grid mode (a 75 x 45 x 37 example runs to its cap of 80 in one
 // start of three), and rounding then grows to 1e-4 of the field within four
@@ -1581,7 +1583,9 @@ int fused_slab(const sgh_plan* p) {
   if (p->cfg.precision == SGH_PRECISION_FP32 || p->cfg.axis_cuda_cores) return 0;
   if (h.prop_corr && phase_branches(p->cfg)) return 0;
   if (vol::col_shape(h.nx, h.ny, h.nz).bytes > vol::COL_SMEM_MAX) return 0;
-  return vol::slab_cluster(h.nx, h.ny, h.nz);
+  const int n = vol::slab_cluster(h.nx, h.ny, h.nz);
+  if (n && p->cfg.precision == SGH_PRECISION_FP64 && !vol::slab_wins(h.nx, h.ny, h.nz, n)) return 0;
+  return n;
 }
 
 // Cluster size of the face-space step, or 0 for the multi-kernel form

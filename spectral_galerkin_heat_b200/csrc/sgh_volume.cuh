@@ -225,6 +225,57 @@ inline int slab_cluster(int nx, int ny, int nz) {
   return best;
 }
 
+// Clocks of one folded pass over nvec vectors on a CTA's 16 warps (64 per MMA and
+// scheduler, two halves a step; see slab_run for the tiles of a task).
+inline long slab_pass_clocks(int N, int nvec) {
+  const int tiles = (nvec + 7) / 8, pairs = (nvec + 15) / 16;
+  const bool two = nvec > 8 && mtiles(N) * pairs >= 8;
+  const int tasks = mtiles(N) * (two ? pairs : tiles);
+  return 128L * ksteps(N) * (two ? 2 : 1) * ((tasks + 3) / 4);
+}
+// Multiplications of one axis pass, padded to the tiles it takes (axis_shape).
+inline double axis_padded(int N, long ncol) {
+  const int tiles[4][2] = {{64, 128}, {64, 64}, {32, 128}, {32, 64}};
+  double w = 0.0;
+  for (int q = 0; q < 4; ++q) {
+    const long r = (N + tiles[q][0] - 1) / tiles[q][0], c = (ncol + tiles[q][1] - 1) / tiles[q][1];
+    w = (double)r * tiles[q][0] * c * tiles[q][1] * N;
+    if (r * c >= AXM_SMS) break;
+  }
+  return w;
+}
+// Whether an FP64 plan's Picard iteration is shorter fused than with one pass per
+// axis. The slab kernels contract half as much, but in waves of the clusters that the
+// GPU holds, and a share of one tile more than its warps divide costs a round. Both
+// sides' us are fitted to 45 of 70 measured volumes (latent heat and property correction;
+// plans with one of the two cross at the same places). The bound leaves room for
+// the fit's error, so that no measured volume is slower fused:
+//   volume          estimate  passes / fused us an iteration
+//   128 x 64 x 32     0.73       76 /   58
+//   256 x 128 x 64    0.67      485 /  337
+//   512 x 128 x 32    0.85      641 /  576
+//   200 x 200 x 100   0.91     1169 / 1011
+//   384 x 192 x 64    0.92     1177 / 1238
+//   320 x 160 x 32    1.22      517 /  540
+//   288 x 144 x 64    1.08      750 /  817
+// Up to 16384 modes, and slabs below 1000, 14 small launches take no longer than five
+// larger ones: 16 x 16 x 8 37 / 41, 32 x 16 x 16 40 / 42, 64 x 32 x 8 44 / 44, 23 x 25
+// x 31 45 / 49; 48 x 24 x 16 48 / 43, 31 x 33 x 17 57 / 48.
+inline bool slab_wins(int nx, int ny, int nz, int n) {
+  const int active[5] = {148, 74, 33, 15, 7};
+  int k = 0;
+  while ((1 << k) < n) ++k;
+  const SlabShape f = slab_shape(nx, ny, n);
+  const double M = 1e-6 * nx * ny * nz;
+  if (M <= 0.016384 || nx * ny < 1000) return false;
+  const double clocks = ((nz + active[k] - 1) / active[k]) *
+                        (2.0 * (slab_pass_clocks(nx, f.R) + slab_pass_clocks(ny, f.C)) + 9000.0);
+  const double fused = 1.6e-3 * clocks + 62.0 * M + 25.0;
+  const double passes = 0.066e-6 * 4.0 * (axis_padded(nx, (long)ny * nz) + axis_padded(ny, (long)nx * nz)) +
+                        119.0 * M + 46.0;
+  return fused <= 0.915 * passes;
+}
+
 struct SlabArgs {
   PointPhys P;
   const double *pxf, *pxi, *pyf, *pyi;

@@ -49,3 +49,21 @@ def test_face_form(nx, ny, cap, cluster):
     counts, err = _against_oracle(ctx)
     assert (counts[1] == 0) == cluster   # a cluster iterates inside its one kernel
     assert err < 1e-10
+
+
+@pytest.mark.parametrize("nx,ny,nz,precision,fused", [
+    (32, 16, 8, "fp64", False), (64, 32, 8, "fp64", False), (48, 24, 16, "fp64", True), (31, 33, 17, "fp64", True),
+    (67, 41, 9, "fp64", True), (100, 17, 33, "fp64", True), (17, 100, 33, "fp64", True), (23, 25, 31, "fp64", False),
+    (320, 160, 8, "fp64", False), (288, 144, 8, "fp64", False), (32, 16, 8, "mixed", True), (320, 160, 8, "mixed", True)])
+@pytest.mark.parametrize("latent_only", [False, True])
+def test_volume_form(nx, ny, nz, precision, fused, latent_only):
+    """Fused slab and column kernels: five launches an iteration (two with latent
+    heat alone) against one pass per axis (14, or 8); mixed plans against
+    the oracle at the 1e-5 bound of their FP32 modes."""
+    from spectral_galerkin_heat_b200 import workloads
+    cfg, path = workloads.nonlinear_raster(nx, ny, nz, steps=3, tol=1e-30, cap=8)
+    if latent_only:
+        cfg["material"].update({"k": 25.0, "Cp": 625.0})
+    counts, err = _against_oracle(make_context(cfg, path), precision=precision)
+    assert (counts[1] == (2 if latent_only else 5)) == fused, counts
+    assert err < (1e-10 if precision == "fp64" else 1e-5)
