@@ -1595,18 +1595,20 @@ int fused_slab(const sgh_plan* p) {
 //   face        chain   one forcing pass    12 iterations
 //   256 x 128      48      110 /  85          458 / 298
 //   384 x 96      120      119 / 104          602 / 449
-//   256 x 224     120      122 / 122          614 / 542
+//   256 x 224     120      122 / 123          614 / 542
 //   256 x 256     128      125 / 132          636 / 584
 //   400 x 128     132      125 / 121          643 / 556
 //   512 x 64      140      128 / 118          658 / 540
 //   288 x 144     144      115 / 129          573 / 600
 //   320 x 160     160      121 / 141          611 / 641
 //   300 x 200     205      126 / 166          640 / 800
-//   16 x 400      104      106 / 111          532 / 528
+//   16 x 400      104      106 / 111          506 / 532
 //   16 x 600      270      136 / 164          722 / 854
-// With one forcing pass per step the chip-wide passes of small faces are the
-// shorter ones (hence the bound by the size), and from 4096 cells a CTA the laser
-// flux, which the chip-wide form spreads over every SM, decides.
+// The chip-wide passes of small faces are the shorter ones, hence the bounds by the
+// size. With one forcing pass per step the laser flux weighs as much as a
+// transform; the chip-wide form spreads it over every SM, a cluster over the CTAs
+// that have rows: 256 x 160 (4096 cells on each of ten) 106 / 110, 200 x 200 (3200
+// on thirteen) 110 / 114, 192 x 192 (3072 on twelve) 109 / 94.
 int face_cluster(const sgh_plan* p) {
   const DevParams& h = p->hp;
   if (!p->face_space || h.has_top_conv || h.has_bottom_conv) return 0;
@@ -1614,8 +1616,8 @@ int face_cluster(const sgh_plan* p) {
   const int n = fold::cluster_size<double>(h.nx, h.ny);
   if (!n) return 0;
   const bool once = p->cfg.max_iter <= 1;
-  if (once && h.S >= 4096 * n) return 0;
-  return fold::face_chain(h.nx, h.ny, n) <= (once ? std::min(140, 84 + h.S / 340) : 140) ? n : 0;
+  if (once && fold::face_shape<double>(h.nx, h.ny, n).R * h.nx > 3100) return 0;
+  return fold::face_chain(h.nx, h.ny, n) <= std::min(140, once ? 84 + h.S / 340 : 80 + h.S / 300) ? n : 0;
 }
 
 // Adds a conditional node of the given type to the graph being captured on

@@ -36,8 +36,8 @@ def _against_oracle(ctx, steps=2, **kw):
 
 
 @pytest.mark.parametrize("nx,ny,cap,cluster", [
-    (64, 32, 1, True), (512, 64, 1, True), (512, 64, 6, True), (256, 256, 1, False), (256, 256, 6, True),
-    (16, 400, 1, False), (16, 400, 6, True), (288, 144, 6, False), (300, 200, 1, False), (1000, 16, 6, False)])
+    (64, 32, 1, True), (512, 64, 1, False), (512, 64, 6, True), (256, 256, 1, False), (256, 256, 6, True),
+    (160, 256, 1, True), (256, 160, 1, False), (16, 400, 1, False), (16, 400, 6, False), (16, 256, 6, True), (288, 144, 6, False), (300, 200, 1, False), (1000, 16, 6, False)])
 def test_face_form(nx, ny, cap, cluster):
     from spectral_galerkin_heat_b200 import workloads
     from spectral_galerkin_heat_b200.laser import StraightTrack
