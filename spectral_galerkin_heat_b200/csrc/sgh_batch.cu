@@ -1930,7 +1930,10 @@ int capture(sgh_batch* B) {
 // slots up to 256 x 128: 1.71 -> 0.86 ms for 6 steps). Mixed: Picard loops up to
 // 32768 elements, where the launches and epilogue latencies of the tensor-core
 // kernels dominate (32 uneven slots, 3 steps of 30 iterations: 7.6 -> 2.4 ms; 4
-// small ragged slots: 10.3 -> 1.9 ms); with one forcing pass per step the
+// small ragged slots: 10.3 -> 1.9 ms), except long thin faces, which give a cluster
+// few tasks of many slices (one slot of 1000 x 16, 12 iterations: 1.17 ms a step on
+// the tensor-core kernels, 1.47 on a cluster; eight of 600 x 32: 1.04 against 1.32;
+// of 512 x 64: 1.06 against 0.97); with one forcing pass per step the
 // tensor-core kernels take all slots of a batch at once and are faster (48
 // serving slots: 1.45 ms against 1.50 with the 64 x 32 faces on clusters, 1.85
 // with every face up to 256 x 128).
@@ -1950,7 +1953,11 @@ int capture(sgh_batch* B) {
 constexpr double CROWD = 3.0;
 int slot_cluster(const sgh_config& c, int precision, double waves) {
   const bool mixed = precision == SGH_PRECISION_MIXED;
-  if (mixed && (c.max_iter <= 1 || (long)c.nx * c.ny > 32768)) return 0;
+  if (mixed) {
+    if (c.max_iter <= 1 || (long)c.nx * c.ny > 32768) return 0;
+    const int n = fold::cluster_size<float>(c.nx, c.ny);
+    if (n && fold::face_chain(c.nx, c.ny, n) > 200) return 0;
+  }
   if (waves > CROWD)
     return mixed ? fold::cluster_size_crowded<float>(c.nx, c.ny) : fold::cluster_size_crowded<double>(c.nx, c.ny);
   return mixed ? fold::cluster_size<float>(c.nx, c.ny) : fold::cluster_size<double>(c.nx, c.ny);

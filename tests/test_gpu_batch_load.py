@@ -52,3 +52,25 @@ def test_slot_alone_in_a_crowd_over_lanes_and_moved(precision):
     lanes.synchronize()
     assert np.array_equal(lanes.modes(COUNT - 1).cpu().numpy(), want)
     lanes.close()
+
+
+@pytest.mark.parametrize("nx,ny,cluster", [(512, 64, True), (64, 512, True), (600, 32, False), (1000, 16, False)])
+def test_long_thin_faces_take_the_shorter_path(nx, ny, cluster):
+    """Mixed Picard slots: a cluster iterates inside its kernel (no launches per
+    iteration); thin faces of very long axes stay on the tensor-core kernels.
+    Either against the FP64 oracle to 1e-4, the bound of the mixed form."""
+    from conftest import rel_l2
+    from oracle.sgh_oracle import OracleSolver
+    from spectral_galerkin_heat_b200.batch import BatchSolver
+    ctx = _ctx(nx, ny)
+    o = OracleSolver(ctx)
+    o.initialize()
+    for k in range(STEPS):
+        o.step(k * ctx.num.dt, ctx.num.dt)
+    b = BatchSolver([ctx], "mixed")
+    assert (b.launch_counts()[1] == 0) == cluster
+    b.start(0, STEPS)
+    b.step(STEPS)
+    assert b.tensor_core_error() == 0
+    assert rel_l2(b.modes(0).double().cpu().numpy(), o.a) < 1e-4
+    b.close()
