@@ -346,6 +346,13 @@ int sgh_dctn(int32_t kind, int32_t ndim, const int32_t* shape, const double* in,
                                    split-BF16 on the tensor cores (slots with a Picard loop and
                                    a face of up to 32768 cells: FP64); FP64 faces and norms */
 
+/* Or'ed into SGH_PRECISION_MIXED: every face of the batch in split-BF16 on the
+ * tensor cores, those of Picard slots too. Slower for a few slots, faster for many
+ * of large faces (12 iterations a step: 16 slots of 256 x 128 1.10 ms against 0.79,
+ * 100 slots 1.78 against 3.31). A slot's bits depend on this choice, and on nothing
+ * else around it. */
+#define SGH_BATCH_TENSOR_FACES 0x100
+
 typedef struct sgh_batch sgh_batch;
 
 typedef struct {

@@ -25,6 +25,7 @@ PICARD_HISTORY_MAX = 4096  # SGH_PICARD_HISTORY_MAX
 ERRORS = {-1: "SGH_ERR_INVALID", -2: "SGH_ERR_CUDA", -3: "SGH_ERR_STATE",
           -4: "SGH_ERR_UNSUPPORTED", -5: "SGH_ERR_WORKSPACE"}
 STEP_STATUS = {0: "converged", 1: "capped", 2: "nonfinite", 3: "tensor_core_timeout"}
+TENSOR_FACES = 0x100   # or'ed into a batch's mixed precision
 PRECISION = {"fp64": 0, "mixed": 1}          # batches and plans
 PLAN_PRECISION = {"fp64": 0, "mixed": 1, "fp32": 2}   # single-instance plans
 BUF = {"modes": 0, "K": 1, "KK": 2, "T_prev": 3, "q_evap_old": 4, "Q_modes": 5,

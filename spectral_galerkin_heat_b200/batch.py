@@ -11,7 +11,8 @@ convection, latent heat or a T-dependent model.
 Slots in FP64, and mixed slots with a Picard loop, whose face fits a
 thread-block cluster run their whole face step in one kernel with FP64
 contractions. The choice depends on the slot alone (its face and its Picard
-cap), so a slot gives the same bits in every batch.
+cap), so a slot gives the same bits in every batch; ``tensor_faces`` puts every
+face of a mixed batch on the tensor cores instead.
 
 ``precision="fp64"`` keeps the modes and K/KK in FP64; ``precision="mixed"``
 stores the modes in FP32 (K and KK formed from FP64 1-D tables), with FP64 face
@@ -53,20 +54,23 @@ class BatchSolver:
     """A bound batch of slots on one device."""
 
     def __init__(self, contexts: Sequence, precision: str = "fp64", device=None,
-                 policy: Optional[dict] = None, stream=None):
+                 policy: Optional[dict] = None, stream=None, tensor_faces: bool = False):
         """``policy``: the kernels' tile policy, ``{"vol_unroll": 2 | 4 | 8,
         "vol_vec": 0 | 1 | 2 | 4}`` (0: the widest vector);
         None takes the autotuner's entry for this grid mix (``tuned.json`` or
         ``SGH_TUNE_TABLE``) and the built-in default without one. ``stream``:
         the CUDA stream of every launch and copy of this batch (default: the
-        device's current stream)."""
+        device's current stream). ``tensor_faces`` (mixed precision): the faces of
+        Picard slots on the tensor cores too, faster for batches of many large
+        ones (from about 24 slots of 256 x 128 or 300 of 128 x 64) and within the
+        same bound."""
         import torch
-        if precision not in _lib.PRECISION:
-            raise ValueError(f"precision must be one of {sorted(_lib.PRECISION)}")
+        code = self._precision_code(precision, tensor_faces)
         if not torch.cuda.is_available():
             raise RuntimeError("BatchSolver needs a CUDA device (no CPU fallback)")
         self.contexts = list(contexts)
         self.precision = precision
+        self.tensor_faces = bool(tensor_faces)
         self.n = len(self.contexts)
         cfgs = (_lib.SghConfig * self.n)()
         for i, ctx in enumerate(self.contexts):
@@ -76,8 +80,7 @@ class BatchSolver:
         self._cfgs = cfgs
         L = _lib.lib()
         h = C.c_void_p()
-        _lib.check("sgh_batch_create", L.sgh_batch_create(cfgs, self.n, _lib.PRECISION[precision],
-                                                          C.byref(h)))
+        _lib.check("sgh_batch_create", L.sgh_batch_create(cfgs, self.n, code, C.byref(h)))
         self._h = h
         if policy is None:
             from .autotune import lookup_batch
@@ -103,7 +106,15 @@ class BatchSolver:
         return C.c_void_p(self.stream.cuda_stream)
 
     @staticmethod
-    def workspace_bytes_for(contexts: Sequence, precision: str = "fp64") -> int:
+    def _precision_code(precision: str, tensor_faces: bool) -> int:
+        if precision not in _lib.PRECISION:
+            raise ValueError(f"precision must be one of {sorted(_lib.PRECISION)}")
+        if tensor_faces and precision != "mixed":
+            raise ValueError("tensor_faces is a choice of mixed-precision batches")
+        return _lib.PRECISION[precision] | (_lib.TENSOR_FACES if tensor_faces else 0)
+
+    @staticmethod
+    def workspace_bytes_for(contexts: Sequence, precision: str = "fp64", tensor_faces: bool = False) -> int:
         """Device bytes a batch of these contexts would bind (computed on the host)."""
         n = len(contexts)
         cfgs = (_lib.SghConfig * n)()
@@ -111,7 +122,8 @@ class BatchSolver:
             cfgs[i] = make_config(ctx, *_picard(ctx))
         L = _lib.lib()
         h = C.c_void_p()
-        _lib.check("sgh_batch_create", L.sgh_batch_create(cfgs, n, _lib.PRECISION[precision], C.byref(h)))
+        _lib.check("sgh_batch_create", L.sgh_batch_create(
+            cfgs, n, BatchSolver._precision_code(precision, tensor_faces), C.byref(h)))
         try:
             nbytes = C.c_uint64()
             _lib.check("sgh_batch_workspace_bytes", L.sgh_batch_workspace_bytes(h, C.byref(nbytes)))
@@ -157,7 +169,11 @@ class BatchSolver:
         info = self.status()[slot]
         return {"modes": self.snapshot(slot, "modes"), "q_evap_old": self.snapshot(slot, "q_evap_old"),
                 "step": int(info.step), "n_steps": int(info.n_steps), "precision": self.precision,
-                "shape": tuple(self.buffer(slot, "modes").shape)}
+                "shape": tuple(self.buffer(slot, "modes").shape), "tensor_faces": self._picard_on_tensor(slot)}
+
+    def _picard_on_tensor(self, slot: int) -> bool:
+        """Whether ``tensor_faces`` decides the bits of ``slot``."""
+        return self.tensor_faces and int(self._cfgs[slot].max_iter) > 1
 
     def import_slot(self, slot: int, state: dict, table) -> None:
         """Continue an exported request in ``slot`` (same grid, physics and
@@ -166,6 +182,8 @@ class BatchSolver:
         on uninterrupted."""
         if state["precision"] != self.precision:
             raise ValueError("a slot state moves between batches of the same precision only")
+        if bool(state.get("tensor_faces", False)) != self._picard_on_tensor(slot):
+            raise ValueError("a Picard slot's state moves between batches of the same tensor_faces only")
         dst = self.buffer(slot, "modes")
         if tuple(dst.shape) != tuple(state["shape"]):
             raise ValueError(f"slot {slot} has modes {tuple(dst.shape)}, the state {state['shape']}")
@@ -299,7 +317,7 @@ class LaneBatch:
     numbers."""
 
     def __init__(self, contexts: Sequence, precision: str = "fp64", lanes: int = 2, device=None,
-                 policy: Optional[dict] = None):
+                 policy: Optional[dict] = None, tensor_faces: bool = False):
         import torch
         self.contexts = list(contexts)
         self.precision = precision
@@ -323,10 +341,11 @@ class LaneBatch:
         for li, m in enumerate(members):
             st = torch.cuda.Stream(dev)
             self.lanes.append(BatchSolver([self.contexts[i] for i in m], precision, device=dev,
-                                          policy=policy, stream=st))
+                                          policy=policy, stream=st, tensor_faces=tensor_faces))
             for local, g in enumerate(m):
                 self.where[g] = (li, local)
         self.policy = self.lanes[0].policy
+        self.tensor_faces = self.lanes[0].tensor_faces
         self.stream = torch.cuda.current_stream(dev)
         self.device = dev
 

@@ -1948,13 +1948,17 @@ int capture(sgh_batch* B) {
 //   4096 elements a CTA  ms    2.62  3.16  4.09  5.31  6.60  11.1  21.6
 //   tensor-core kernels  ms    6.57  7.71  7.78  8.38  8.94  11.2  17.2
 // FP64 crosses from 2048 to 4096 at the same place (64 slots 4.33 against 4.44,
-// 128: 8.33 against 7.45). Past some 10 waves the tensor-core kernels would be the
-// faster ones for mixed slots; they are not taken there, for the reason above.
+// 128: 8.33 against 7.45). For mixed slots the tensor-core kernels are the faster
+// ones from some 10 waves on, and from fewer where every face is large (12
+// iterations a step, clusters / tensor cores, us: 16 slots of 256 x 128 793 / 1103,
+// 32 1425 / 1157, 100 3310 / 1783; 64 of 128 x 64 411 / 922, 400 2102 / 1796). They
+// are not taken by the load, for the reason above: a caller that fills a batch
+// with large Picard slots asks for them (SGH_BATCH_TENSOR_FACES).
 constexpr double CROWD = 3.0;
-int slot_cluster(const sgh_config& c, int precision, double waves) {
+int slot_cluster(const sgh_config& c, int precision, bool tensor_faces, double waves) {
   const bool mixed = precision == SGH_PRECISION_MIXED;
   if (mixed) {
-    if (c.max_iter <= 1 || (long)c.nx * c.ny > 32768) return 0;
+    if (tensor_faces || c.max_iter <= 1 || (long)c.nx * c.ny > 32768) return 0;
     const int n = fold::cluster_size<float>(c.nx, c.ny);
     if (n && fold::face_chain(c.nx, c.ny, n) > 200) return 0;
   }
@@ -1964,10 +1968,10 @@ int slot_cluster(const sgh_config& c, int precision, double waves) {
 }
 
 // Times the cluster slots of a batch fill the chip, at FACE_SHARE elements a CTA.
-double slot_waves(const sgh_config* cfgs, int n, int precision) {
+double slot_waves(const sgh_config* cfgs, int n, int precision, bool tensor_faces) {
   double e = 0;
   for (int i = 0; i < n; ++i)
-    if (slot_cluster(cfgs[i], precision, 0)) e += (double)cfgs[i].nx * cfgs[i].ny;
+    if (slot_cluster(cfgs[i], precision, tensor_faces, 0)) e += (double)cfgs[i].nx * cfgs[i].ny;
   return e / (148.0 * fold::FACE_SHARE);
 }
 
@@ -1988,6 +1992,8 @@ int sgh_batch_create(const sgh_config* cfgs, int32_t n, int32_t precision, sgh_b
   if (!cfgs || !out) return bfail(SGH_ERR_INVALID, "null argument");
   *out = nullptr;
   if (n < 1 || n > 65536) return bfail(SGH_ERR_INVALID, "slot count must be in [1, 65536]");
+  const bool tensor_faces = precision == (SGH_PRECISION_MIXED | SGH_BATCH_TENSOR_FACES);
+  if (tensor_faces) precision = SGH_PRECISION_MIXED;
   if (precision != SGH_PRECISION_FP64 && precision != SGH_PRECISION_MIXED)
     return bfail(SGH_ERR_INVALID, "precision must be SGH_PRECISION_FP64 or SGH_PRECISION_MIXED");
   sgh_batch* B = new sgh_batch();
@@ -2030,13 +2036,13 @@ int sgh_batch_create(const sgh_config* cfgs, int32_t n, int32_t precision, sgh_b
     moff += 2LL * kv.first * kv.first;
   }
   B->mat_elems = moff;
-  const double waves = slot_waves(cfgs, n, precision);
+  const double waves = slot_waves(cfgs, n, precision, tensor_faces);
   std::map<int, long long> mplane;
   if (precision == SGH_PRECISION_MIXED) {
     long long po = 0;
     std::map<int, int> wide;  // lengths of the slots on the tensor-core path
     for (int i = 0; i < n; ++i)
-      if (!slot_cluster(cfgs[i], precision, waves)) wide[cfgs[i].nx] = wide[cfgs[i].ny] = 1;
+      if (!slot_cluster(cfgs[i], precision, tensor_faces, waves)) wide[cfgs[i].nx] = wide[cfgs[i].ny] = 1;
     for (auto& kv : wide) {
       // per N: forward, inverse in 128-row chunks (the A operand of the
       // y-pass and the B operand of the x-pass alike)
@@ -2070,7 +2076,7 @@ int sgh_batch_create(const sgh_config* cfgs, int32_t n, int32_t precision, sgh_b
     sl.mx = (int)mats[c.nx];
     sl.my = (int)mats[c.ny];
     sl.nblk = cdivl(sl.S, BT);
-    sl.cl = slot_cluster(c, precision, waves);
+    sl.cl = slot_cluster(c, precision, tensor_faces, waves);
     if (sl.cl)
       for (int q = 0; q < 4; ++q) sl.fold[q] = fold_at(q < 2 ? c.nx : c.ny) + (q & 1) * (long long)fold::pack_doubles(q < 2 ? c.nx : c.ny);
     sl.rblk0 = B->tot_rblk;

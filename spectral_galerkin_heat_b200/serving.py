@@ -127,7 +127,8 @@ class ServingEngine:
     memory demand (default: equal). ``lanes`` > 1 splits the slots over that
     many batches on their own CUDA streams, stepped concurrently
     (:class:`LaneBatch`), so one lane's latency-bound face transforms overlap
-    another's bandwidth-bound volume pass. Slot capacity: starting from one slot per
+    another's bandwidth-bound volume pass. ``tensor_faces`` is that of the batches.
+    Slot capacity: starting from one slot per
     class, slots go to the class with the lowest slots/weight ratio while the
     batch workspace fits in ``memory_fraction`` of the free device memory and
     stays within ``max_slots`` slots per class.
@@ -139,17 +140,18 @@ class ServingEngine:
                  keep_modes: bool = False, max_chunk: int = 64,
                  batch_factory: Optional[Callable] = None, mem_info: Optional[Callable] = None,
                  slot_bytes: Optional[Callable] = None, adaptive: bool = False,
-                 rebalance_interval: float = 1.0, lanes: int = 1):
+                 rebalance_interval: float = 1.0, lanes: int = 1, tensor_faces: bool = False):
         if batch_factory is None:
             import torch
             if not torch.cuda.is_available():
                 raise RuntimeError("ServingEngine needs a CUDA device (no CPU fallback)")
             if int(lanes) > 1:
-                batch_factory = functools.partial(LaneBatch, lanes=int(lanes))
+                batch_factory = functools.partial(LaneBatch, lanes=int(lanes), tensor_faces=tensor_faces)
             else:
-                batch_factory = BatchSolver
+                batch_factory = functools.partial(BatchSolver, tensor_faces=tensor_faces)
             mem_info = mem_info or torch.cuda.mem_get_info
-        self._slot_bytes_fn = slot_bytes or (lambda ctx: BatchSolver.workspace_bytes_for([ctx], precision))
+        self._slot_bytes_fn = slot_bytes or (lambda ctx: BatchSolver.workspace_bytes_for(
+            [ctx], precision, tensor_faces))
         self._batch_factory = batch_factory
         self._mem_info = mem_info
         self.precision = precision

@@ -74,3 +74,38 @@ def test_long_thin_faces_take_the_shorter_path(nx, ny, cluster):
     assert b.tensor_core_error() == 0
     assert rel_l2(b.modes(0).double().cpu().numpy(), o.a) < 1e-4
     b.close()
+
+
+def test_tensor_faces_is_the_callers_choice():
+    """Picard slots on the tensor cores by request: within 1e-4 of the oracle, the
+    same bits alone and among others, and no state moves between the two kinds
+    of batch (their bits differ); FP64 batches refuse the choice."""
+    from conftest import rel_l2
+    from oracle.sgh_oracle import OracleSolver
+    from spectral_galerkin_heat_b200.batch import BatchSolver
+    ctxs = [_ctx(128, 64), _ctx(64, 33), _ctx(100, 60)]
+    o = OracleSolver(ctxs[0])
+    o.initialize()
+    for k in range(STEPS):
+        o.step(k * ctxs[0].num.dt, ctxs[0].num.dt)
+
+    def run(cs):
+        b = BatchSolver(cs, "mixed", tensor_faces=True)
+        for i in range(len(cs)):
+            b.start(i, STEPS)
+        b.step(STEPS)
+        assert b.tensor_core_error() == 0 and b.launch_counts()[1] > 0
+        return b
+
+    mix, alone = run(ctxs), run(ctxs[:1])
+    assert rel_l2(mix.modes(0).double().cpu().numpy(), o.a) < 1e-4
+    assert np.array_equal(mix.modes(0).cpu().numpy(), alone.modes(0).cpu().numpy())
+    plain = BatchSolver(ctxs[:1], "mixed")
+    table = plain.laser_table(ctxs[0], 0.0, STEPS)
+    with pytest.raises(ValueError, match="tensor_faces"):
+        plain.import_slot(0, alone.export_slot(0), table)
+    alone.import_slot(0, mix.export_slot(0), table)
+    for b in (mix, alone, plain):
+        b.close()
+    with pytest.raises(ValueError, match="tensor_faces"):
+        BatchSolver(ctxs[:1], "fp64", tensor_faces=True)
