@@ -794,6 +794,8 @@ k_face_run(const DevParams* __restrict__ P, Ctrl* ctrl, fold::FaceShape f, fold:
   const unsigned lim = ctrl->wait_limit ? ctrl->wait_limit : umma::WAIT_LIMIT;
   const bool ok = fold::face_operands(f, J, fr_sh, bar, lim, ctrl->stall_test != 0, &ctrl->umma_err);
   const fold::FaceResult r = fold::face_step<double, KEEPM>(f, J, fr_sh, !ok);
+  if (J.max_iter == 0)  // no iteration, no evaporation: the next step's warm start is none (:512)
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < f.nx * f.ny; i += gridDim.x * blockDim.x) J.qev[i] = 0.0;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     sgh_step_out o;
     o.T_surface_max = r.tmax;
