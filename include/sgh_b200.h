@@ -384,7 +384,9 @@ int sgh_batch_workspace_bytes(const sgh_batch* batch, uint64_t* bytes);
  * slots start inactive. Synchronises the stream. */
 int sgh_batch_bind(sgh_batch* batch, void* workspace, uint64_t bytes, void* stream);
 /* (Re)start a slot: initial condition, laser table (n_steps entries, device),
- * optional per-step metrics table (device, may be NULL). Async. */
+ * optional per-step metrics table (device, may be NULL). Modes that the caller
+ * writes over the initial condition before the next step count (see
+ * sgh_batch_buffer). Async. */
 int sgh_batch_slot_start(sgh_batch* batch, int32_t slot, const sgh_laser* lasers_dev, int32_t n_steps,
                          sgh_step_out* outs_dev, void* stream);
 /* Stop a slot (it is skipped by later steps). Async. */
@@ -410,6 +412,15 @@ int sgh_batch_status(const sgh_batch* batch, sgh_batch_slot_info* out, void* str
 /* Device pointer / size of a slot buffer: SGH_BUF_MODES, SGH_BUF_K, SGH_BUF_KK
  * (element type FP64 or FP32 by precision), SGH_BUF_Q_EVAP_OLD, SGH_BUF_SURFACE (FP64). */
 int sgh_batch_buffer(const sgh_batch* batch, int32_t slot, int32_t which, void** ptr, uint64_t* bytes);
+/* A start forms the first step's face sums with the initial condition, as long as
+ * nobody else can write the modes: once sgh_batch_buffer has given out a pointer
+ * to a slot's SGH_BUF_MODES, its first step after a start forms them from the
+ * volume. SGH_BUF_MODES | SGH_BUF_WATCHED is for callers that only read, or that
+ * call sgh_batch_slot_modes_written after each write: that pointer changes
+ * nothing, and the call makes the next step form the sums from the modes as they
+ * are then. Async. */
+#define SGH_BUF_WATCHED 0x100
+int sgh_batch_slot_modes_written(sgh_batch* batch, int32_t slot, void* stream);
 /* *err = nonzero once a bounded wait of the batch's face or volume kernels
  * expired (the affected face pass, or the whole face step of a slot that runs
  * in a cluster, wrote no results; such a slot's step ends SGH_STEP_NONFINITE). Synchronises the stream. */

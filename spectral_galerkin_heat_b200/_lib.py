@@ -28,6 +28,7 @@ STEP_STATUS = {0: "converged", 1: "capped", 2: "nonfinite", 3: "tensor_core_time
 TENSOR_FACES = 0x100   # or'ed into a batch's mixed precision
 PRECISION = {"fp64": 0, "mixed": 1}          # batches and plans
 PLAN_PRECISION = {"fp64": 0, "mixed": 1, "fp32": 2}   # single-instance plans
+BUF_WATCHED = 0x100   # or'ed into a batch slot's modes buffer
 BUF = {"modes": 0, "K": 1, "KK": 2, "T_prev": 3, "q_evap_old": 4, "Q_modes": 5,
        "surface": 6, "scratch": 7, "box_T_prev": 8, "box_Q_prev": 9, "box_Bx": 10,
        "box_By": 11, "box_Bz": 12}
@@ -47,7 +48,7 @@ EXPORTED = (
     "sgh_batch_create", "sgh_batch_destroy", "sgh_batch_workspace_bytes", "sgh_batch_bind",
     "sgh_batch_slot_start", "sgh_batch_slot_stop", "sgh_batch_slot_resume", "sgh_batch_step", "sgh_batch_step_eager",
     "sgh_batch_status",
-    "sgh_batch_buffer", "sgh_batch_launch_counts", "sgh_batch_volume_pass", "sgh_batch_error",
+    "sgh_batch_buffer", "sgh_batch_slot_modes_written", "sgh_batch_launch_counts", "sgh_batch_volume_pass", "sgh_batch_error",
     "sgh_batch_set_wait_limit", "sgh_batch_set_policy", "sgh_dct2_bf16x3_workspace_bytes",
     "sgh_dct2_bf16x3",
 )
@@ -169,6 +170,7 @@ def lib() -> C.CDLL:
             "sgh_batch_step": ([vp, i32, vp], C.c_int),
             "sgh_batch_step_eager": ([vp, vp], C.c_int),
             "sgh_batch_status": ([vp, C.POINTER(SghBatchSlotInfo), vp], C.c_int),
+            "sgh_batch_slot_modes_written": ([vp, i32, vp], C.c_int),
             "sgh_batch_buffer": ([vp, i32, i32, C.POINTER(vp), u64p], C.c_int),
             "sgh_batch_error": ([vp, C.POINTER(i32), vp], C.c_int),
             "sgh_batch_set_wait_limit": ([vp, C.c_uint32, i32, vp], C.c_int),

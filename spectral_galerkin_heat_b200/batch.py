@@ -101,6 +101,7 @@ class BatchSolver:
                                                       nbytes.value, self._s()))
         self._tables = [None] * self.n
         self._outs = [None] * self.n
+        self._fresh = {}   # slots started and not stepped yet -> the workspace's version at their start
 
     def _s(self):
         return C.c_void_p(self.stream.cuda_stream)
@@ -160,6 +161,29 @@ class BatchSolver:
         _lib.check("sgh_batch_slot_start", _lib.lib().sgh_batch_slot_start(
             self._h, int(slot), C.c_void_p(table.data_ptr()), int(n_steps),
             C.c_void_p(outs.data_ptr()) if outs is not None else None, self._s()))
+        self._fresh[slot] = self._version()
+
+    def _version(self):
+        """Counter that torch raises with every write to the workspace or a view of
+        it; None where torch does not keep one (inference tensors)."""
+        return None if self.workspace.is_inference() else self.workspace._version
+
+    def modes_written(self, slot: int) -> None:
+        """Tell the batch that ``slot``'s modes were written between its start and
+        its next step. Only needed for writes that torch does not see (a captured
+        graph's, another library's) through a view taken before the start: torch
+        writes, and views taken after the start, are noticed."""
+        _lib.check("sgh_batch_slot_modes_written", _lib.lib().sgh_batch_slot_modes_written(
+            self._h, int(slot), self._s()))
+        self._fresh.pop(slot, None)
+
+    def _settle(self) -> None:
+        """Before a step: report the started slots whose modes may have been written."""
+        if self._fresh:
+            now = self._version()
+            for slot in [s for s, v in self._fresh.items() if v is None or v != now]:
+                self.modes_written(slot)
+            self._fresh.clear()
 
     def export_slot(self, slot: int) -> dict:
         """The state a slot carries between steps, as device copies: its modes
@@ -169,7 +193,7 @@ class BatchSolver:
         info = self.status()[slot]
         return {"modes": self.snapshot(slot, "modes"), "q_evap_old": self.snapshot(slot, "q_evap_old"),
                 "step": int(info.step), "n_steps": int(info.n_steps), "precision": self.precision,
-                "shape": tuple(self.buffer(slot, "modes").shape), "tensor_faces": self._picard_on_tensor(slot)}
+                "shape": tuple(self._view(slot, "modes").shape), "tensor_faces": self._picard_on_tensor(slot)}
 
     def _picard_on_tensor(self, slot: int) -> bool:
         """Whether ``tensor_faces`` decides the bits of ``slot``."""
@@ -184,12 +208,16 @@ class BatchSolver:
             raise ValueError("a slot state moves between batches of the same precision only")
         if bool(state.get("tensor_faces", False)) != self._picard_on_tensor(slot):
             raise ValueError("a Picard slot's state moves between batches of the same tensor_faces only")
-        dst = self.buffer(slot, "modes")
+        dst = self._view(slot, "modes")
         if tuple(dst.shape) != tuple(state["shape"]):
             raise ValueError(f"slot {slot} has modes {tuple(dst.shape)}, the state {state['shape']}")
+        before = self._version()
         with _torch_stream(self.stream):
             dst.copy_(state["modes"])
             self.buffer(slot, "q_evap_old").copy_(state["q_evap_old"])
+        self._fresh.pop(slot, None)
+        for s, v in self._fresh.items():   # these two writes are not to a started slot
+            self._fresh[s] = self._version() if v == before else v
         self._tables[slot] = table
         self._outs[slot] = None
         _lib.check("sgh_batch_slot_resume", _lib.lib().sgh_batch_slot_resume(
@@ -201,10 +229,12 @@ class BatchSolver:
 
     def step(self, n_steps: int = 1) -> None:
         """Advance every active slot by ``n_steps`` steps (asynchronous)."""
+        self._settle()
         _lib.check("sgh_batch_step", _lib.lib().sgh_batch_step(self._h, int(n_steps), self._s()))
 
     def step_eager(self) -> None:
         """One step with the kernels launched one by one (profilers, debugging)."""
+        self._settle()
         _lib.check("sgh_batch_step_eager", _lib.lib().sgh_batch_step_eager(self._h, self._s()))
 
     def status(self):
@@ -231,11 +261,19 @@ class BatchSolver:
 
     def buffer(self, slot: int, name: str):
         """torch view of a slot buffer: ``modes``, ``K``, ``KK`` (FP64 or FP32),
-        ``q_evap_old``, ``surface`` (FP64)."""
+        ``q_evap_old``, ``surface`` (FP64). Modes may be written; what is written
+        between a start and the next step replaces the initial condition (see
+        :meth:`modes_written`)."""
+        if name == "modes" and slot in self._fresh:
+            self.modes_written(slot)
+        return self._view(slot, name)
+
+    def _view(self, slot: int, name: str):
         import torch
         ptr, nb = C.c_void_p(), C.c_uint64()
         _lib.check("sgh_batch_buffer", _lib.lib().sgh_batch_buffer(
-            self._h, int(slot), _lib.BUF[name], C.byref(ptr), C.byref(nb)))
+            self._h, int(slot), _lib.BUF[name] | (_lib.BUF_WATCHED if name == "modes" else 0), C.byref(ptr),
+            C.byref(nb)))
         off = ptr.value - self.workspace.data_ptr()
         c = self._cfgs[slot]
         vol = name in ("modes", "K", "KK")
@@ -256,11 +294,11 @@ class BatchSolver:
 
     def fetch(self, slot: int, name: str) -> np.ndarray:
         """Host copy of a slot buffer (synchronises the stream)."""
-        return self.buffer(slot, name).to("cpu").numpy()
+        return self._view(slot, name).to("cpu").numpy()
 
     def snapshot(self, slot: int, name: str):
         """Device copy of a slot buffer (the slot may be reused afterwards)."""
-        return self.buffer(slot, name).clone()
+        return self._view(slot, name).clone()
 
     def volume_pass(self) -> None:
         """The step's volume pass alone over every active slot (timing, profiling)."""
@@ -396,6 +434,10 @@ class LaneBatch:
 
     def modes(self, slot):
         return self.buffer(slot, "modes")
+
+    def modes_written(self, slot):
+        b, local = self._l(slot)
+        b.modes_written(local)
 
     def fetch(self, slot, name):
         b, local = self._l(slot)

@@ -287,11 +287,13 @@ __global__ void __launch_bounds__(BT) kb_weights(BView v, const R* KK, R* Wtt, R
 // the zero mode is set, so the first step's face sums and norm are one term
 // each: they are written here, with the volume pass's arithmetic, instead of
 // read from the whole volume before the first step (48 serving slots started
-// and stepped five times: 1441 -> 1386 us). Four modes per thread.
+// and stepped five times: 1441 -> 1386 us). They serve the first step where the
+// modes are still those written here (`sums`; see sgh_batch_buffer). Four modes per
+// thread.
 template <class R>
 __global__ void __launch_bounds__(BT)
 kb_slot_start(BView v, int s, R* a, const R* K, const R* KK, double* q_evold, double* sigma, R* Zt, R* Yt,
-              double* part_n1, const sgh_laser* table, int n_steps, sgh_step_out* outs) {
+              double* part_n1, const sgh_laser* table, int n_steps, sgh_step_out* outs, int sums) {
   constexpr bool TAB = sizeof(R) == 4;
   const BSlot& sl = v.slot[s];
   const long long i = (long long)blockIdx.x * BT + threadIdx.x;
@@ -345,9 +347,13 @@ kb_slot_start(BView v, int s, R* a, const R* K, const R* KK, double* q_evold, do
     st.iters = 0;
     st.done = 1;
     st.iter = 0;
-    st.pass1_ready = 1;
+    st.pass1_ready = sums;
   }
 }
+
+// The slot's modes were written from outside: the next step forms their face
+// sums from the volume.
+__global__ void kb_sums_stale(BView v, int s) { v.st[s].pass1_ready = 0; }
 
 __global__ void kb_slot_stop(BView v, int s) { v.st[s].active = 0; }
 
@@ -1668,6 +1674,10 @@ struct sgh_batch {
   long long fold_elems = 0;
   size_t o_clist = 0, o_cshape = 0, o_fold = 0;
   size_t xa_bytes = 0, mp_bytes = 0, x1_bytes = 0;
+  // Slots whose face sums were written at their start and not used yet, and slots
+  // whose modes a caller holds a pointer to: what it writes counts in the first step.
+  std::vector<uint8_t> fresh;
+  mutable std::vector<uint8_t> lent;
   int vec = 1;  // columns per thread of the volume passes
   int vol_unroll = 4;  // z-planes per load round of the volume passes (2, 4 or 8)
   std::vector<std::pair<int, long long>> mplane_list;  // (N, byte offset of the forward plane)
@@ -1975,6 +1985,17 @@ double slot_waves(const sgh_config* cfgs, int n, int precision, bool tensor_face
   return e / (148.0 * fold::FACE_SHARE);
 }
 
+// Before a step: slots started since the last one whose modes have been lent out
+// since, too.
+int settle_started(sgh_batch* B, cudaStream_t s) {
+  for (int i = 0; i < B->n; ++i) {
+    if (B->fresh[i] && B->lent[i]) kb_sums_stale<<<1, 1, 0, s>>>(B->view(), i);
+    B->fresh[i] = 0;
+  }
+  SGB_CK(cudaGetLastError());
+  return SGH_OK;
+}
+
 struct LayoutB {
   size_t off = 0;
   size_t take(size_t bytes) {
@@ -2000,6 +2021,8 @@ int sgh_batch_create(const sgh_config* cfgs, int32_t n, int32_t precision, sgh_b
   B->n = n;
   B->precision = precision;
   B->cfg.assign(cfgs, cfgs + n);
+  B->fresh.assign(n, 0);
+  B->lent.assign(n, 0);
   std::map<int, long long> mats;
   for (int i = 0; i < n; ++i) {
     const sgh_config& c = cfgs[i];
@@ -2361,12 +2384,22 @@ int sgh_batch_slot_start(sgh_batch* B, int32_t slot, const sgh_laser* lasers_dev
   if (B->precision == SGH_PRECISION_MIXED)
     kb_slot_start<float><<<g, BT, 0, s>>>(B->view(), slot, B->f(B->o_a), nullptr, nullptr, B->d(B->o_qevold),
                                           B->d(B->o_sigma), B->f(B->o_Zt), B->f(B->o_Yt), B->d(B->o_pn1),
-                                          lasers_dev, n_steps, outs_dev);
+                                          lasers_dev, n_steps, outs_dev, B->lent[slot] ? 0 : 1);
   else
     kb_slot_start<double><<<g, BT, 0, s>>>(B->view(), slot, B->d(B->o_a), B->d(B->o_K), B->d(B->o_KK),
                                            B->d(B->o_qevold), B->d(B->o_sigma), B->d(B->o_Zt), B->d(B->o_Yt),
-                                           B->d(B->o_pn1), lasers_dev, n_steps, outs_dev);
+                                           B->d(B->o_pn1), lasers_dev, n_steps, outs_dev, B->lent[slot] ? 0 : 1);
   SGB_CK(cudaGetLastError());
+  B->fresh[slot] = B->lent[slot] ? 0 : 1;
+  return SGH_OK;
+}
+
+int sgh_batch_slot_modes_written(sgh_batch* B, int32_t slot, void* stream) {
+  if (!B || !B->bound) return bfail(SGH_ERR_STATE, "batch is not bound");
+  if (slot < 0 || slot >= B->n) return bfail(SGH_ERR_INVALID, "slot out of range");
+  kb_sums_stale<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(B->view(), slot);
+  SGB_CK(cudaGetLastError());
+  B->fresh[slot] = 0;
   return SGH_OK;
 }
 
@@ -2395,6 +2428,7 @@ int sgh_batch_step(sgh_batch* B, int32_t n_steps, void* stream) {
   if (n_steps < 0) return bfail(SGH_ERR_INVALID, "n_steps must be >= 0");
   if (n_steps == 0) return SGH_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (const int rc = settle_started(B, s)) return rc;
   kb_run_setup<<<1, 1, 0, s>>>(B->view(), n_steps);
   SGB_CK(cudaGetLastError());
   SGB_CK(cudaGraphLaunch(B->exec, s));
@@ -2404,6 +2438,7 @@ int sgh_batch_step(sgh_batch* B, int32_t n_steps, void* stream) {
 int sgh_batch_step_eager(sgh_batch* B, void* stream) {
   if (!B || !B->bound) return bfail(SGH_ERR_STATE, "batch is not bound");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (const int rc = settle_started(B, s)) return rc;
   kb_run_setup<<<1, 1, 0, s>>>(B->view(), 1);
   const bool mixed = B->precision == SGH_PRECISION_MIXED;
   if (mixed) enqueue_pre<float>(B, s, 0, 0);
@@ -2445,7 +2480,8 @@ int sgh_batch_buffer(const sgh_batch* B, int32_t slot, int32_t which, void** ptr
   const BSlot& sl = B->slots[slot];
   const size_t e = B->elem();
   size_t off, nb;
-  switch (which) {
+  if (which == SGH_BUF_MODES) B->lent[slot] = 1;
+  switch (which & ~SGH_BUF_WATCHED) {
     case SGH_BUF_MODES: off = B->o_a + e * sl.vol; nb = e * sl.V; break;
     case SGH_BUF_K:
       if (B->precision == SGH_PRECISION_MIXED)
