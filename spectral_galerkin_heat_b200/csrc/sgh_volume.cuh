@@ -36,7 +36,7 @@ constexpr int COL_THREADS = 256;
 enum { SLAB_INIT, SLAB_TRIAL, SLAB_TRIAL_RELAX, SLAB_RELAX, SLAB_QM };
 enum { COL_LATENT, COL_TEMP, COL_STENCIL, COL_COMMIT };
 
-__device__ __forceinline__ int pos_of(int m, int n) { return (m & 1) ? half_up(n) + (m >> 1) : (m >> 1); }
+__host__ __device__ __forceinline__ int pos_of(int m, int n) { return (m & 1) ? half_up(n) + (m >> 1) : (m >> 1); }
 
 // Where a pass puts its results: output p of vector v at row(p)[v * vs], for v <
 // nv; pair: two neighbouring vectors (vs = 1) may be stored as one 16-byte word.
