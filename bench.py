@@ -32,8 +32,8 @@ transforms, FP64 face fields, norms and coefficient tables, FP32 face sums).
 ``--workload raster`` is the full nonlinear FP64 case (128 x 64 x 32 modes,
 T-dependent properties, latent heat, evaporation + convection, Picard to
 1e-8) through ``B200SpectralSolver``: ``value`` from the device-resident step
-graph (``sgh_run``), ``e2e`` through ``step(t, dt)``, the DCT axis pass as the
-roofline kernel. ``--workload track`` is the 64 x 32 x 16 straight track.
+graph (``sgh_run``), ``e2e`` through ``step(t, dt)``, ``roofline`` of the loop's
+fused kernels (of the DCT axis pass where a plan runs one pass per axis). ``--workload track`` is the 64 x 32 x 16 straight track.
 
 ``--impl reference`` times the CPU implementation alone (rank 0) on the same
 workload and prints the same JSON line with ``"impl": "reference"``.
@@ -66,8 +66,8 @@ L2_FLUSH_BYTES = 256 << 20
 # (288 slots, 467,927,040 active modes) read 1.976 GB and wrote 1.968 GB
 # (--cache-control none); traffic scales with the modes of the same class mix.
 NCU_VOLUME_TRAFFIC_PER_MODE = (1975895808 + 1967578624) / 467927040
-# the raster workload's dominant kernel (k_axis) was captured on the same
-# 128x64x32 case: 2.14 MB for one contiguous-axis pass (field resident in L2)
+# one axis pass (k_axis) of a 128x64x32 field, for plans that run one pass per axis:
+# 2.14 MB for a contiguous-axis pass (field resident in L2)
 NCU_TRAFFIC_BYTES = 2.14e6
 # the box workload's box passes (one reconstruction + one projection) from an
 # ncu capture of the same case; None until captured
@@ -331,7 +331,7 @@ def run_b200(args, rank, world, local_rank):
         roof = _box_roofline(s, flush, stream, dev)
         s.finalize()
     else:
-        roof = _axis_roofline(s, flush, stream, dev)
+        roof = _loop_roofline(s, dev_ms, iters, dev) or _axis_roofline(s, flush, stream, dev)
         s.finalize()
 
     # ---- end to end through the public API ----------------------------------
@@ -527,6 +527,33 @@ def _box_roofline(s, flush, stream, dev):
             # bytes each pass reads and writes once, both directions
             "hbm_gbs_algorithmic": 8.0 * 2 * (nz * S + 2 * zb * S + 2 * zb * ny * xb + zb * yb * xb)
             / (ms * 1e-3) / 1e9}
+
+
+def _loop_roofline(s, step_ms, iters, dev):
+    """FP64 contraction work of the timed steps of a plan whose loop runs in cluster
+    or fused kernels, over the steps' own time; None for one pass per axis. The
+    work is that of the halved contractions those kernels do."""
+    pre, per_it, post = s.launch_counts()
+    nz, ny, nx = s.state.shape
+    if per_it == 0:
+        # per step: the forcing and every iteration forward, every iteration and the
+        # commit inverse; a face transform is S (nx + ny) flops
+        kernel = "k_fs_volume + k_face_run (one cluster runs the whole face step)"
+        flops = sum((1 + n) * 2.0 * nx * ny * (nx + ny) for n in iters)
+        note = "latency of the cluster's passes and barriers, one face on at most 16 SMs"
+    elif per_it in (2, 5):
+        # per iteration, each axis: forward and inverse once (latent heat), twice with the correction
+        sets = 2 if per_it == 2 else 4
+        kernel = "k_column + k_slab (fused volume form)"
+        flops = sum(n * sets * float(nx * ny * nz) * (nx + ny + nz) for n in iters)
+        note = "operand reads from shared memory, cluster barriers, launch boundaries"
+    else:
+        return None
+    peak = _fp64_peak(dev)
+    achieved = flops / (step_ms * 1e-3) / 1e12
+    return {"kernel": kernel, "bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+            "frac": achieved / peak, "peak_source": "measured here: cuBLAS DGEMM 4096^3, best of 10",
+            "traffic": None, "algorithmic_flops_per_step": flops / len(iters), "note": note}
 
 
 def _axis_roofline(s, flush, stream, dev):
@@ -1184,8 +1211,9 @@ def run_outputs(args, rank, world, local_rank):
             return Kn.reconstruct_temperature_DCT(d, st).to("cpu")
         e2e_ms = timed(e2e)
         nodal_bytes = 8 * (nx * ny * nz + (nx + 1) * (ny + 1) * (nz + 1))
-        nodal_flop = 2.0 * ((nx + 1) * nx * ny * nz + (ny + 1) * ny * nz * (nx + 1)
-                            + (nz + 1) * nz * (ny + 1) * (nx + 1))
+        # passes z, y, x, each halved by the cosine's symmetry
+        nodal_flop = 1.0 * ((nz + 1) * nz * ny * nx + (ny + 1) * ny * (nz + 1) * nx
+                            + (nx + 1) * nx * (ny + 1) * (nz + 1))
         t0 = time.perf_counter()
         n_cpu = 0
         while time.perf_counter() - t0 < min(args.cpu_budget, 10.0) or n_cpu < 1:
@@ -1210,13 +1238,13 @@ def run_outputs(args, rank, world, local_rank):
                        "l2": "flushed between timed launches (256 MB write)"},
             "e2e": {"value": 1e3 / big["nodal_e2e_ms"], "unit": "1/s", "h2d_bytes_per_step": 8 * 512 * 256 * 64,
                     "d2h_bytes_per_step": 8 * 513 * 257 * 65},
-            "roofline": {"kernel": "3 axis passes of the node field (FP64 tensor cores)", "bound": "fp64",
+            "roofline": {"kernel": "k_sym (3 halved passes of the node field, FP64 tensor cores)", "bound": "fp64",
                          "achieved": big["nodal_fp64_tflops"], "peak": fp64, "unit": "TFLOP/s",
                          "frac": big["nodal_fp64_tflops"] / fp64,
                          "peak_source": "measured here: cuBLAS DGEMM 4096^3, best of 10", "traffic": None,
                          "hbm_gbs_min_traffic": big["nodal_gbs_min_traffic"], "hbm_peak": hbm,
                          "hbm_peak_source": hbm_kind,
-                         "note": "FP64 contraction work bounds it (dense N x (N+1) passes), not HBM"},
+                         "note": "FP64 contraction work bounds it (halved N x (N+1) passes), not HBM"},
             "cpu_baseline": {"value": 1e3 / big["nodal_cpu_reference_algorithm_ms"], "unit": "1/s",
                              "cores": os.cpu_count(), "kind": "port",
                              "sample": "the reference's weighted DCT-I (scipy, all threads) on the same modes"}}
