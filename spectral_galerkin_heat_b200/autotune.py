@@ -93,11 +93,20 @@ def tune(ctx, candidates: Iterable[int] = CANDIDATES, steps: int = 10, warmup: i
          kernels: Iterable[int] = KERNELS) -> Dict:
     """Time each (threshold, kernel) pair on ``ctx``'s step; returns the choice
     and the per-candidate ms per Picard iteration and per step (keys
-    ``"<threshold>|<axis_cuda_cores>"``)."""
+    ``"<threshold>|<axis_cuda_cores>"``). A loop without axis passes (a cluster or
+    the fused volume form) does not depend on the threshold, a cluster's not on
+    the kernel either: those are timed once."""
     res = {}
     for kern in kernels:
+        per_iter = None
         for c in candidates:
-            res[(int(c), int(kern))] = _time_one(ctx, int(c), int(kern), steps, warmup)
+            r = _time_one(ctx, int(c), int(kern), steps, warmup)
+            per_iter = r.pop("launches_per_iter")
+            res[(int(c), int(kern))] = r
+            if per_iter <= 5:
+                break
+        if per_iter == 0:
+            break
     best = min(res, key=lambda ck: res[ck]["ms_per_iter"])
     return {"axis_min_ctas": best[0], "axis_cuda_cores": best[1],
             "candidates": {f"{c}|{k}": v for (c, k), v in res.items()},
@@ -125,8 +134,9 @@ def _time_one(ctx, c: int, kern: int, steps: int, warmup: int) -> Dict:
     ms = a.elapsed_time(b)
     recs = s.decode_outs(outs.cpu().numpy().tobytes(), warmup + steps)[warmup:]
     iters = max(1, sum(max(1, r.n_iter) for r in recs))
+    per_iter = s.launch_counts()[1]   # 0: one cluster kernel; 2 or 5: fused; more: one pass per axis
     s.finalize()
-    return {"ms_per_step": ms / steps, "ms_per_iter": ms / iters, "iters": iters}
+    return {"ms_per_step": ms / steps, "ms_per_iter": ms / iters, "iters": iters, "launches_per_iter": per_iter}
 
 
 def tune_table(contexts: Dict[str, object], out: Optional[str] = None, **kw) -> Dict:

@@ -67,3 +67,15 @@ def test_volume_form(nx, ny, nz, precision, fused, latent_only):
     counts, err = _against_oracle(make_context(cfg, path), precision=precision)
     assert (counts[1] == (2 if latent_only else 5)) == fused, counts
     assert err < (1e-10 if precision == "fp64" else 1e-5)
+
+
+def test_tuner_times_only_what_differs():
+    """A loop without axis passes has no threshold to tune, a cluster's no kernel."""
+    from spectral_galerkin_heat_b200 import workloads
+    from spectral_galerkin_heat_b200.autotune import tune
+    track = make_context(*workloads.straight_track(steps=8))
+    r = tune(track, candidates=(1, 132), steps=3, warmup=1)
+    assert list(r["candidates"]) == ["1|0"] and r["axis_cuda_cores"] == 0
+    raster = make_context(*workloads.nonlinear_raster(64, 32, 16, steps=8, cap=5))
+    r = tune(raster, candidates=(1, 132), steps=3, warmup=1)
+    assert sorted(r["candidates"]) == ["132|1", "1|0", "1|1"]
