@@ -298,15 +298,13 @@ int sgh_box_window(sgh_plan* plan, int32_t* i0, void* stream);
 int sgh_picard_history(sgh_plan* plan, double* out, int32_t cap, int32_t* n_iter, void* stream);
 
 /* Bound of the data waits of a plan's slab kernels (the fused volume form) and
- * of its face-space cluster kernel: at
- * most `polls` mbarrier polls (0 = the default, 2^22) before the kernel records
- * the error and waits for its copies in flight (with the default bound). The
- * step's Picard loop then ends (the cluster kernel writes no results at all) and
- * the step reports SGH_STEP_TC_TIMEOUT,
- * as do later ones until the plan is bound again. stall_test = 1 makes every
- * such wait run out (needs polls > 0), so that a test can drive the error path
- * without a fault; 0 for normal stepping. No reference counterpart.
- * Synchronises the stream. */
+ * of its face-space cluster kernel: at most `polls` mbarrier polls (0 = the
+ * default, 2^22) before the kernel records the error and waits for its copies in
+ * flight (with the default bound). The step's Picard loop then ends (the cluster
+ * kernel writes no results at all) and the step reports SGH_STEP_TC_TIMEOUT, as
+ * do that plan's later ones. stall_test = 1 makes every such wait run out (needs
+ * polls > 0), so that a test can drive the error path without a fault; 0 for
+ * normal stepping. No reference counterpart. Synchronises the stream. */
 int sgh_plan_set_wait_limit(sgh_plan* plan, uint32_t polls, int32_t stall_test, void* stream);
 
 /* out (nz_box, ny_box, nx_box) = the temperature of modes on the fine box at
