@@ -29,7 +29,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -779,7 +778,7 @@ k_fs_volume(Ctrl* ctrl, sgh_laser laser, const sgh_laser* table, sgh_step_out* o
 template <bool KEEPM>
 __global__ void __launch_bounds__(fold::FACE_THREADS, 1)
 k_face_run(const DevParams* __restrict__ P, Ctrl* ctrl, fold::FaceShape f, fold::FaceJob<double> J,
-           cudaGraphConditionalHandle h_steps, int in_graph) {
+           cudaGraphConditionalHandle h_steps, int in_graph, unsigned wait_limit, bool stall_test) {
   extern __shared__ __align__(128) double fr_sh[];
   __shared__ uint64_t bar[2];
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
@@ -791,8 +790,7 @@ k_face_run(const DevParams* __restrict__ P, Ctrl* ctrl, fold::FaceShape f, fold:
   J.ly = L.y;
   J.shift_x = laser_shift(L.vx, P->dt, P->dx, f32);
   J.shift_y = laser_shift(L.vy, P->dt, P->dy, f32);
-  const unsigned lim = ctrl->wait_limit ? ctrl->wait_limit : umma::WAIT_LIMIT;
-  const bool ok = fold::face_operands(f, J, fr_sh, bar, lim, ctrl->stall_test != 0, &ctrl->umma_err);
+  const bool ok = fold::face_operands(f, J, fr_sh, bar, wait_limit, stall_test, &ctrl->umma_err);
   const fold::FaceResult r = fold::face_step<double, KEEPM>(f, J, fr_sh, !ok);
   if (J.max_iter == 0)  // no iteration, no evaporation: the next step's warm start is none (:512)
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < f.nx * f.ny; i += gridDim.x * blockDim.x) J.qev[i] = 0.0;
@@ -873,6 +871,8 @@ struct sgh_plan {
   };
   std::vector<PlaneSpec> plane_specs;
   std::vector<UmmaPlane> planes;
+  unsigned wait_limit = umma::WAIT_LIMIT;  // polls of the slab and cluster kernels' data waits
+  bool stall_test = false;                 // they first wait on a barrier that nothing completes
   bool bound_planes = false;
   size_t ws_need = 0;
   char* ws = nullptr;
@@ -1229,7 +1229,7 @@ void enqueue_face_run(sgh_plan* p, cudaStream_t s, cudaGraphConditionalHandle h_
   const fold::FaceShape f = fold::face_shape<double>(p->hp.nx, p->hp.ny, p->cluster);
   auto go = [&](auto kernel) {
     SGH_CK_VOID(fold::launch_cluster(kernel, f.n, f.n, fold::threads_for(f), f.bytes, true, s, p->P(), p->ctrl(), f,
-                                     face_job(p), h_steps, in_graph));
+                                     face_job(p), h_steps, in_graph, p->wait_limit, p->stall_test));
   };
   if (f.keep & fold::FACE_M) go(k_face_run<true>);
   else go(k_face_run<false>);
@@ -1337,6 +1337,8 @@ void enqueue_slab(sgh_plan* p, const double* in, double* out, cudaStream_t s, cu
   q.ctrl = p->ctrl();
   q.h_picard = h_picard;
   q.in_graph = in_graph;
+  q.wait_limit = p->wait_limit;
+  q.stall_test = p->stall_test;
   if (f.keep)
     SGH_CK_VOID(fold::launch_cluster(vol::k_slab<MODE, true>, f.n * h.nz, f.n, vol::SLAB_THREADS, f.bytes, true, s, f, q));
   else
@@ -2165,17 +2167,22 @@ int sgh_step_eager(sgh_plan* p, const sgh_laser* laser, sgh_step_out* out, void*
 }
 
 int sgh_plan_set_wait_limit(sgh_plan* p, uint32_t polls, int32_t stall_test, void* stream) {
+  AxisPolicy policy(p ? p->cfg.axis_min_ctas : 0, p ? p->cfg.axis_cuda_cores : 0, plan_mixed(p), umma_err_of(p),
+                    plan_fp32(p), planes_of(p), nplanes_of(p));
   if (!p) return fail(SGH_ERR_INVALID, "null argument");
   if (!p->bound) return fail(SGH_ERR_STATE, "plan is not bound");
   if (stall_test && polls == 0) return fail(SGH_ERR_INVALID, "the wait test needs an explicit poll bound");
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const unsigned v[2] = {polls, stall_test ? 1u : 0u};
-  static_assert(offsetof(Ctrl, stall_test) == offsetof(Ctrl, wait_limit) + sizeof(unsigned),
-                "wait_limit and stall_test are adjacent");
-  SGH_CK(cudaMemcpyAsync(reinterpret_cast<char*>(p->ctrl()) + offsetof(Ctrl, wait_limit), v, sizeof(v),
-                         cudaMemcpyHostToDevice, s));
-  SGH_CK(cudaStreamSynchronize(s));
-  return SGH_OK;
+  SGH_CK(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
+  p->wait_limit = polls ? polls : umma::WAIT_LIMIT;
+  p->stall_test = stall_test != 0;
+  // the bound is an argument of the kernels: the step graph is captured again
+  SGH_CK(cudaGraphExecDestroy(p->exec));
+  p->exec = nullptr;
+  SGH_CK(cudaGraphDestroy(p->graph));
+  p->graph = nullptr;
+  const int rc = capture(p);
+  if (rc) p->bound = false;  // no graph to step with
+  return rc;
 }
 
 int sgh_run(sgh_plan* p, const sgh_laser* lasers_dev, int32_t n_steps, sgh_step_out* outs_dev, void* stream) {

@@ -67,8 +67,6 @@ struct Ctrl {
   int hist_cap;
   unsigned tickets;  // CTAs of the current relaxation done (back to 0 after it)
   int umma_err;  // a bounded wait of one of the plan's kernels ran out
-  unsigned wait_limit;  // polls of the slab and cluster kernels' waits (0: umma::WAIT_LIMIT)
-  int stall_test;       // 1: they first wait on a barrier that nothing completes
 };
 
 // ---------------------------------------------------------------------------
@@ -379,8 +377,10 @@ __device__ __forceinline__ void block_max_sum(double& m, double& s, double* sh) 
 
 // Convergence test of one Picard iteration (solvers/spectral.py:464-499):
 // err = sqrt(sum res^2 / n) / max(sqrt(sum a_old^2 / n), 1e-9). Updates the
-// control block; nonzero when the loop stops.
+// control block; nonzero when the loop stops, as it does once a bounded wait of the
+// step's kernels has run out.
 __device__ __forceinline__ int converge_test(const DevParams& P, Ctrl* ctrl, double s0, double s1) {
+  if (ctrl->umma_err) s0 = nan("");
   const double rms_d = sqrt(s0 / P.n_elements);
   const double rel = rms_d / fmax(sqrt(s1 / P.n_elements), 1e-9);
   const int it = ctrl->iter + 1;

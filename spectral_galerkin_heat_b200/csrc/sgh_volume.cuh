@@ -291,33 +291,32 @@ struct SlabArgs {
   Ctrl* ctrl;             // QM: skipped when no iteration ran; *RELAX: convergence test
   cudaGraphConditionalHandle h_picard;
   int in_graph;
+  unsigned wait_limit;    // polls of the operand wait
+  bool stall_test;        // it first waits on a barrier that nothing completes
 };
 
 // Waits for the packed matrices' copies on bar[0], at most lim polls a thread. A
 // thread whose wait ran out (or, with `stall`, that first waited on bar[1], which
-// nothing completes) records it in *err and *expired and waits for the copies with
-// the full bound, so that none outlives the CTA.
-__device__ __forceinline__ void slab_operands(uint64_t* bar, unsigned lim, bool stall, int* err, int* expired) {
+// nothing completes) records it in *err and waits for the copies with the full
+// bound, so that none outlives the CTA.
+__device__ __forceinline__ void slab_operands(uint64_t* bar, unsigned lim, bool stall, int* err) {
   bool ok = !stall || umma::mbar_wait_bounded(&bar[1], 0u, lim);
   ok = ok && umma::mbar_wait_bounded(&bar[0], 0u, lim);
   if (!ok) {
     atomicExch(err, 1);
-    *expired = 1;
     umma::mbar_wait_bounded(&bar[0], 0u, umma::WAIT_LIMIT);
   }
 }
 
 // KEEP: the packed matrices are in shared memory (f.keep), else read from L2.
-// An expired wait is recorded in ctrl->umma_err: the step reports
-// SGH_STEP_TC_TIMEOUT, and its relaxations write NaN partials, so that the Picard
-// loop ends there.
+// An expired wait is recorded in ctrl->umma_err: the convergence test then ends the
+// Picard loop, and the step reports SGH_STEP_TC_TIMEOUT.
 template <int MODE, bool KEEP>
 __global__ void __launch_bounds__(SLAB_THREADS, 1) k_slab(SlabShape f, SlabArgs q) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ __align__(128) double sl_sh[];
   __shared__ uint64_t bar[2];
-  __shared__ int expired;  // a wait of this CTA ran out
   __shared__ double red[2 * (SLAB_THREADS / 32)];
   constexpr int NW = SLAB_THREADS / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -336,7 +335,6 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) k_slab(SlabShape f, SlabArgs 
   const double* pyi = KEEP ? sl_sh + f.o_m + nyp + 2 * nxp : q.pyi;
   // The packed matrices never change: their copies start before the wait for
   // the previous kernel.
-  if (tid == 0) expired = 0;
   if (KEEP && tid == 0) {
     double* o = sl_sh + f.o_m;
     umma::mbar_init(&bar[0], 1);
@@ -349,13 +347,10 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) k_slab(SlabShape f, SlabArgs 
     umma::bulk_g2s(o + nyp + 2 * nxp, q.pyi, 8 * nyp, &bar[0]);
   }
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
-  // read here, used far below: the flag of the step's earlier kernels, the waits' bound
-  const int err0 = q.ctrl->umma_err, stall = q.ctrl->stall_test;
-  const unsigned limit = q.ctrl->wait_limit;
   if (MODE == SLAB_QM && q.ctrl->iter <= 0) {  // the same for every CTA
     if (KEEP) {
       __syncthreads();
-      slab_operands(bar, limit ? limit : umma::WAIT_LIMIT, stall != 0, &q.ctrl->umma_err, &expired);  // no copy outlives the CTA
+      slab_operands(bar, q.wait_limit, q.stall_test, &q.ctrl->umma_err);  // no copy outlives the CTA
     }
     return;
   }
@@ -388,7 +383,7 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) k_slab(SlabShape f, SlabArgs 
   }
   if (KEEP) {
     __syncthreads();  // the barriers are initialised
-    slab_operands(bar, limit ? limit : umma::WAIT_LIMIT, stall != 0, &q.ctrl->umma_err, &expired);
+    slab_operands(bar, q.wait_limit, q.stall_test, &q.ctrl->umma_err);
   }
   cl.sync();  // the slab is loaded; every CTA runs before any remote write
   double s0 = 0.0, s1 = 0.0;
@@ -471,7 +466,7 @@ __global__ void __launch_bounds__(SLAB_THREADS, 1) k_slab(SlabShape f, SlabArgs 
     __shared__ int last;
     block_sum2<SLAB_THREADS>(s0, s1, red);
     if (tid == 0) {
-      q.partials[2 * blockIdx.x] = err0 || expired ? nan("") : s0;
+      q.partials[2 * blockIdx.x] = s0;
       q.partials[2 * blockIdx.x + 1] = s1;
       __threadfence();
       last = atomicAdd(&q.ctrl->tickets, 1u) == gridDim.x - 1;
