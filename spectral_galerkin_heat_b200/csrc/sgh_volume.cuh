@@ -8,7 +8,7 @@
 //   slab kernels (k_slab)   one cluster per z-mode: y and x transforms of one
 //     slab, forward, then the modal update, then inverse, with the two
 //     transposes through distributed shared memory;
-//   column kernels (k_column) 32 or 64 (y, x) columns per CTA with all of z:
+//   column kernels (k_column) 16 or 32 (y, x) columns per CTA with all of z:
 //     z-inverse, pointwise physics, z-forward.
 // With latent heat and the property correction:
 //   B = xy-inverse of the iterate (kept between iterations)
@@ -496,8 +496,8 @@ struct ColShape {
 inline ColShape col_shape(int nx, int ny, int nz) {
   ColShape f;
   f.nx = nx; f.ny = ny; f.nz = nz;
-  // 16 columns per CTA (two vector tiles): the pointwise physics wants every
-  // warp slot of the SMs
+  // 16 columns per CTA (two vector tiles) up to 14,208 columns: the pointwise physics
+  // wants every warp slot of the SMs; 32 where that many CTAs fill them anyway
   f.cc = (long)nx * ny <= 16 * 148 * 6 ? 16 : 32;
   f.ld = fold::face_ld(f.cc);
   f.bytes = (nz + std::max(nz, COL_THREADS / f.cc)) * f.ld * 8;
