@@ -792,7 +792,7 @@ k_face_run(const DevParams* __restrict__ P, Ctrl* ctrl, fold::FaceShape f, fold:
   J.shift_y = laser_shift(L.vy, P->dt, P->dy, f32);
   const bool ok = fold::face_operands(f, J, fr_sh, bar, wait_limit, stall_test, &ctrl->umma_err);
   const fold::FaceResult r = fold::face_step<double, KEEPM>(f, J, fr_sh, !ok);
-  if (J.max_iter == 0)  // no iteration, no evaporation: the next step's warm start is none (:512)
+  if (J.max_iter == 0 && r.status != SGH_STEP_NONFINITE)  // no iteration, no evaporation: no warm start either (:512)
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < f.nx * f.ny; i += gridDim.x * blockDim.x) J.qev[i] = 0.0;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     sgh_step_out o;
@@ -1595,7 +1595,7 @@ int fused_slab(const sgh_plan* p) {
 // Cluster size of the face-space step, or 0 for the multi-kernel form
 // (convection, reduced precision, faces too large for a cluster, and those whose
 // passes on the cluster's few SMs take longer than the chip-wide ones and their
-// launches). Measured over 42 faces, us a step, one pass per axis / cluster:
+// launches). Measured over 44 faces, us a step, one pass per axis / cluster:
 //   face        chain   one forcing pass    12 iterations
 //   256 x 128      48      110 /  85          458 / 298
 //   384 x 96      120      119 / 104          602 / 449

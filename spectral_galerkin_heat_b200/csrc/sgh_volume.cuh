@@ -247,7 +247,7 @@ inline double axis_padded(int N, long ncol) {
 // Whether an FP64 plan's Picard iteration is shorter fused than with one pass per
 // axis. The slab kernels contract half as much, but in waves of the clusters that the
 // GPU holds, and a share of one tile more than its warps divide costs a round. Both
-// sides' us are fitted to 45 of 70 measured volumes (latent heat and property correction;
+// sides' us are fitted to 45 of 75 measured volumes (latent heat and property correction;
 // plans with one of the two cross at the same places). The bound leaves room for
 // the fit's error, so that no measured volume is slower fused:
 //   volume          estimate  passes / fused us an iteration
